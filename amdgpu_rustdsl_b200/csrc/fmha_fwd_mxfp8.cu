@@ -4,10 +4,11 @@
 // one (batch, head) and a key range [key_lo, key_hi), out = softmax2(q k^T) v with
 //   q k^T  : e4m3 x e4m3 with one E8M0 scale per 32 elements of the head dim on both sides (block-scaled tensor-core MMA),
 //   softmax: base 2, no extra scale (the host folds log2(e)/sqrt(128) into Q before quantisation, tests/gpu/ref_host.cpp:238),
-//            online over 128-key tiles with a lazily moved reference: the reference only moves when a row maximum passes it by
-//            more than a threshold, and then O and the row sum are rescaled (crates/amdgpu-tile/src/softmax.rs:179-243);
+//            online over the keys with a lazily moved reference: the reference only moves when a row maximum passes it by
+//            more than a threshold (crates/amdgpu-tile/src/softmax.rs:179-243; there O and the row sum are then rescaled, here P carries the
+//            difference as its block scale);
 //            sequences under 4 tiles move the reference on every tile (crates/amdgpu-stage/src/attention/state.rs:73-77),
-//   P      : requantised to e4m3 before P V, and the row sum adds the *quantised* P (crates/amdgpu-tile/src/reduce.rs:163-173),
+//   P      : requantised to e4m3 (long sequences: with one E8M0 per row and 32 keys) before P V, and the row sum adds the *quantised* P (crates/amdgpu-tile/src/reduce.rs:163-173),
 //   out    : O * v_descale / l as bf16 (state.rs:79-82), or for the split kernel the normalised f32 partial plus a base-2
 //            log-sum-exp per row (block3.rs:291-356).
 //
@@ -28,17 +29,18 @@
 //   warp  3    V producer: TMA loads of the V ring (K is freed after Q K^T, V after P V, so the two rings run apart), and the K scale
 //              gathers of the tiles with an odd counter.
 //   warps 4-11 softmax, two warpgroups: warpgroup p works on the tiles with counter g = p (mod 2). Thread r of a group owns query row
-//              r = TMEM lane r: it reads the row's 128 scores with one tensor-memory round trip and hands the S buffer back at once,
-//              takes the row's reference from the group of the previous tile through an 8-byte shared-memory slot {value, tile
-//              counter}, converts in place, writes P (packed e4m3) with tcgen05.st, and rescales O in TMEM on the rare tiles that move
-//              the reference.
+//              r = TMEM lane r: it reads the row's 128 scores from tensor memory and hands the S buffer back at once, converts block by
+//              block of 32 keys with the block's own reference, writes P (packed e4m3) with tcgen05.st and, when they change, the
+//              row's block scales to shared memory. The references travel between the groups through 8-byte shared-memory slots
+//              {value, tile counter}, off the critical path.
 //   warps 12-15 epilogue, one warpgroup: takes an item's O and row sums out of tensor memory when its last P V is done, hands the
 //              columns back (the next item's first P V waits for that), normalises, stages the tile in shared memory and stores it
 //              with TMA (bf16 output, or the split kernel's partial), while the softmax warpgroups are on the next item's tiles.
 //              Merges the two halves of an item cut between a pair of CTAs; in the fused instantiations merges a row block's partials.
 //   Every thread starts with 128 registers; the service warps then keep 56, the softmax warps take 176 and the epilogue warps 104
 //   (setmaxnreg: the roles' shares must come out of the CTA's launch allocation).
-// TMEM columns: S0 [0,128) S1 [128,256) O [256,384) L [384,400) P0 [400,432) P1 [432,464) SFQ [464,468) SFK0 [468,472) SFK1 [472,476).
+// TMEM columns: S0 [0,128) S1 [128,256) O [256,384) L [384,400) P0 [400,432) P1 [432,464) SFQ [464,468) SFK0 [468,472) SFK1 [472,476)
+// SFP [476,480) SFV [480,488).
 #include "kernels.h"
 #include "ptx_sm100.cuh"
 
@@ -86,16 +88,19 @@ constexpr uint32_t kColS0 = 0, kColS1 = 128, kColO = 256, kColL = 384, kColP0 = 
 constexpr uint32_t kTmemCols = 512;
 
 // P = 2^(s - ref + kPOffset): the row's reference maps to 2^kPOffset.
-// Long sequences (>= 4 key tiles): the reference is an integer, ceil(tile maximum), and is left alone while a tile's maximum stays
-// within kLazyThreshold binades above it, so P <= 2^(5 + 3.5) = 362 < 448 never saturates e4m3. Integer references make every
-// rescale an exact power of two, so the same keys give the same P mantissas whatever the reference: a KV split and the unsplit
-// kernel then differ only by f32 summation order.
+// Long sequences (>= 4 key tiles): the reference is an integer, ceil(block maximum), and is left alone while a block's maximum stays
+// within kLazyThreshold binades above it, so P <= 2^(5 + 3.5) = 362 < 448 never saturates e4m3. Integer references differ by exact powers of
+// two, so the same keys give the same P mantissas whatever the reference: a KV split and the unsplit kernel then differ only by f32
+// summation order (and where P is subnormal).
 // Short sequences move the reference to the tile's own maximum on every tile whose maximum is less than kFollowWindow binades
 // below it (so every tile's largest P is exactly 2^kPOffset, which is what keeps the error on sharply peaked rows at the level of
 // the reference's short-sequence recipe: thr 120/512 vs target 131/512, crates/amdgpu-tile/src/softmax.rs:26-30).
 constexpr float kPOffset = 5.0f;
 constexpr float kLazyThreshold = 3.5f;
 constexpr float kFollowWindow = 11.0f;
+// Long sequences: O and L are in units of the row's base and a tile's P carries 2^(reference - base) as its block scale. The products stay far
+// inside f32 for 2^(8.5 + 60) x 2^8.8 (the largest e4m3 V) x 2^20 keys.
+constexpr float kRebase = 60.0f;
 constexpr uint32_t kFlagCausal = 0x8u;   // FMHA_MXFP8_FLAG_CAUSAL: selects the kCausal instantiations
 constexpr uint32_t kFlagF32Partials = 0x10u;   // FMHA_MXFP8_FLAG_F32_PARTIALS: the split kernel's partial rows are f32, not f16
 constexpr uint32_t kFlagNoTailSplit = 0x20u;   // FMHA_MXFP8_FLAG_NO_TAIL_SPLIT: never cut the last round's items in two
@@ -112,18 +117,18 @@ struct SmemLayout {
     static constexpr uint32_t ostage = ones + 4096;
     static constexpr uint32_t sfq = ostage + 2 * 16384;
     static constexpr uint32_t sfk = sfq + 2 * kSfBytes;
-    // [tile counter % 4][row 128] x {reference bits, tile counter}. Four slots per row, not two: a softmax warpgroup goes from an item's
-    // last tile straight on to the next item's first, which reads no reference, so it may publish tile g while the other group has yet to
-    // read what tile g - 2 left for its tile g - 1
+    // [tile counter % 8][row 128] x {reference bits, tile counter}. A group that publishes tile g + 6 has finished g + 4, so P V of g + 2 and
+    // with it that of g + 1 is done, so the other group is past its tile g + 1 and has read slot g: six slots are enough
     static constexpr uint32_t sfv = sfk + kStages * kSfBytes;    // V block scales of a key tile (extension), same 32 x 16-byte pattern as the K scales
     static constexpr uint32_t sf_one = sfv + kStages * kSfBytes;  // 512 bytes of E8M0 1.0: the factors of P and of the ones columns
     static constexpr uint32_t xref = sf_one + kSfBytes;
     // [item ordinal % 4][row 128]: the row's reference after the item's last tile, for the epilogue warpgroup. Four slots and a write
     // behind the wait for this parity's previous P V: with one-tile items a softmax group is otherwise two items ahead of the epilogue
-    static constexpr uint32_t xfin = xref + 4 * 128 * 8;
+    static constexpr uint32_t xfin = xref + 8 * 128 * 8;
     static constexpr uint32_t xstat = xfin + 4 * 128 * 4;         // [row 128] x {row sum, reference} of the partner's half item (launches as pairs)
     static constexpr uint32_t xlse = xstat + 128 * 8;             // fused merge: [row 128][split 8] log-sum-exps of the block being merged
-    static constexpr uint32_t bars = xlse + 128 * 8 * 4;
+    static constexpr uint32_t sfp = xlse + 128 * 8 * 4;          // P block scales, one buffer per softmax group, same 32 x 16-byte pattern
+    static constexpr uint32_t bars = sfp + 2 * kSfBytes;
     // barriers (8 bytes each): q_full[2], q_empty[2], k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages], s_full[2], s_free[2],
     // p_full[2], o_done[2], o_free, o_full, four unused, peer_rdy, peer_data
     static constexpr uint32_t n_bars = 4 + 4 * kStages + 16;
@@ -169,9 +174,9 @@ __device__ __forceinline__ uint32_t p_word(uint32_t s0, uint32_t s1, uint32_t s2
 // tensor rate, so two of every four P values are produced on the FMA pipe instead, straight as e4m3 bit patterns:
 // byte = rne(8 (x + 7)) with x = log2 P, i.e. exponent field = floor(x) + 7 and a mantissa that is linear in the fraction of x
 // (the piecewise-linear exp2 the reference uses for all of P, crates/amdgpu-tile/src/reduce.rs:94-113, docs/vendor-spec.md:271-281).
-// fma.sat clamps t = s / 32 + c to [0, 1] = bytes 0..256 (so -inf scores give 0), and adding 2^15 leaves rne(256 t) in the low byte of the
-// sum. The additions (this one, and the shift in front of the exp2 of the other two values) are done two at a time (add.f32x2); the
-// two-wide fma has no saturating form, so the clamped fma stays one per value.
+// The rounding, the clamp at zero and the packing are one conversion: 8 (x + 7) 2^-24 is a subnormal f16 whose bit pattern is the byte, and
+// cvt.relu takes everything below (-inf scores too) to 0. So two values cost one two-wide fma and one conversion, against two clamped fma, an
+// addition and a permute for doing the rounding in f32; the additions in front of the exp2 of the other two are also done two at a time.
 // The linear mantissa overestimates 2^frac by 3.97 % on average; kFastBias shifts x so that the two kinds of P values agree on
 // average, otherwise mixing them in one row sum would bias the weights.
 constexpr float kFastBias = 0.0562f;
@@ -191,10 +196,20 @@ __device__ __forceinline__ void mul2(uint32_t& a, uint32_t& b, float c) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(p), "l"(q));
     asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(p));
 }
-__device__ __forceinline__ uint32_t fast_p_sat(uint32_t s, float c) {   // s / 32 + c clamped to [0, 1]
-    float t;
-    asm("fma.rn.sat.f32 %0, %1, 0f3D000000, %2;" : "=f"(t) : "f"(__uint_as_float(s)), "f"(c));
-    return __float_as_uint(t);
+// a = a x + c, b = b x + c in one instruction
+__device__ __forceinline__ void fma2(uint32_t& a, uint32_t& b, float x, float c) {
+    unsigned long long p, q, r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "r"(a), "r"(b));
+    asm("mov.b64 %0, {%1, %1};" : "=l"(q) : "f"(x));
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(c));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p) : "l"(p), "l"(q), "l"(r));
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(p));
+}
+// max(a, 0) in the low and max(b, 0) in the high half, as f16 (subnormals kept)
+__device__ __forceinline__ uint32_t cvt_relu_f16x2(float a, float b) {
+    uint32_t h;
+    asm("cvt.rn.relu.f16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(b), "f"(a));
+    return h;
 }
 __device__ __forceinline__ void st_shared_v2(uint32_t addr, uint32_t a, uint32_t b) {
     asm volatile("st.volatile.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
@@ -213,14 +228,18 @@ __device__ __forceinline__ void stamp_t(float* trace, int role, int tile, int sl
     if (kTrace && trace != nullptr && tile < 32) reinterpret_cast<long long*>(trace + kStampBase)[(role * 32 + tile) * 8 + slot] = clock64();
 }
 
-// O columns [col, col + 32) of this thread's lane *= f
-__device__ __forceinline__ void scale_tmem32(uint32_t taddr, float f) {
-    uint32_t o[32];
-    tmem_ld32(taddr, o);
+// O columns [col, col + 64) of this thread's lane *= f
+__device__ __forceinline__ void scale_tmem64(uint32_t taddr, float f) {
+    uint32_t a[32], b[32];
+    tmem_ld32(taddr, a);
+    tmem_ld32(taddr + 32, b);
     tmem_wait_ld();
 #pragma unroll
-    for (int c = 0; c < 32; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * f);
-    tmem_st32(taddr, o);
+    for (int c = 0; c < 32; c += 2) mul2(a[c], a[c + 1], f);
+    tmem_st32(taddr, a);
+#pragma unroll
+    for (int c = 0; c < 32; c += 2) mul2(b[c], b[c + 1], f);
+    tmem_st32(taddr + 32, b);
 }
 
 // One unit of work of the persistent kernel: 128 query rows of one (batch, head) against the key range of one split.
@@ -336,7 +355,6 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t n_items = p.n_work, stride = gridDim.x;   // the work units this grid walks (whole items, and halves of the last round's)
     // kLazy: the long-sequence recipe, chosen by the launcher from the whole sequence's tile count, also in a split (block3.rs:180-184)
     constexpr bool lazy = kLazy;
-    constexpr float thr = lazy ? kLazyThreshold : -kFollowWindow;
     const bool cta_traced = kTrace && p.trace != nullptr && blockIdx.x == 0;   // diagnostics cover the first item of CTA 0 = logical block (0,0,0)
 
     // Programmatic dependent launch: the next launch in the stream (if it asks for it, as this library's own launches do) may be
@@ -366,15 +384,15 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         mbar_init(bar_peer_data, kRows);
         fence_mbar_init();
     }
-    if (kVbs && threadIdx.x >= 256 && threadIdx.x < 384) {
+    if ((kLazy || kVbs) && threadIdx.x >= 256 && threadIdx.x < 384) {
         reinterpret_cast<uint32_t*>(smem_gen + SmemLayout::sf_one)[threadIdx.x - 256] = 0x7F7F7F7Fu;
         fence_proxy_async_smem();
     }
     if (threadIdx.x < 256) {
         for (int i = 0; i < 4; ++i) reinterpret_cast<uint32_t*>(smem_gen + SmemLayout::ones)[threadIdx.x + 256 * i] = 0x38383838u;
-        // the 512 reference hand-over slots start with a tile counter no tile has
-        reinterpret_cast<uint2*>(smem_gen + SmemLayout::xref)[threadIdx.x] = make_uint2(0u, 0xFFFFFFFFu);
-        reinterpret_cast<uint2*>(smem_gen + SmemLayout::xref)[threadIdx.x + 256] = make_uint2(0u, 0xFFFFFFFFu);
+        // the 1024 reference hand-over slots start with a tile counter no tile has
+        for (int i = 0; i < 4; ++i) reinterpret_cast<uint2*>(smem_gen + SmemLayout::xref)[threadIdx.x + 256 * i] = make_uint2(0u, 0xFFFFFFFFu);
+        reinterpret_cast<uint32_t*>(smem_gen + SmemLayout::sfp)[threadIdx.x] = 0x7F7F7F7Fu;
         fence_proxy_async_smem();
     }
     if (warp == kMmaWarp) {
@@ -668,11 +686,14 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             // V block scales (extension): the same MMA as kind::mxf8f6f4.block_scale, P's factors a constant 1.0, V's one E8M0 per 32 keys and column
             const uint32_t idesc_pv_bs = idesc_mxf8_block_scaled(128, 144, 0, 1, 0, 0);
             const uint32_t t_sfp = tmem + kColSfP, t_sfv = tmem + kColSfV;
-            if (kVbs && elect_one_sync()) {   // the constant factors, once: P's four columns and the ones columns' (rows 128..143 of the B factors)
+            constexpr bool kScaled = kLazy || kVbs;   // P V as the block-scaled kind
+            if (kScaled && elect_one_sync()) {   // the constant factors, once: the ones columns' (rows 128..143 of the B factors), V's without block scales, P's in the short recipe
                 const uint64_t d1 = make_smem_desc(smem_base + SmemLayout::sf_one, 0, 128, kSwizzleNone);
-                tmem_cp_sf(t_sfp, d1);
+                if (!kLazy) tmem_cp_sf(t_sfp, d1);
+                if (!kVbs) tmem_cp_sf(t_sfv, d1);
                 tmem_cp_sf(t_sfv + 4, d1);
             }
+            const uint64_t dsfp0 = make_smem_desc(smem_base + SmemLayout::sfp, 0, 128, kSwizzleNone);
             uint32_t g = 0, n = 0, ph = 0;
             int st = 0;
             bool ok = true;
@@ -695,8 +716,9 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             // MN-major B: 8-key groups 1024 B apart; the second 128-byte-wide atom (columns 128..) is the tile of ones
                             const uint32_t v_addr = v_smem + st * kTileBytes + kb * 4096;
                             const uint64_t dv = make_smem_desc(v_addr, ones_smem - v_addr, 1024, kSwizzle128B);
-                            if (kVbs) {
-                                if (kb == 0) tmem_cp_sf(t_sfv, make_smem_desc(smem_base + SmemLayout::sfv + st * kSfBytes, 0, 128, kSwizzleNone));
+                            if (kScaled) {
+                                if (kLazy && kb == 0) tmem_cp_sf(t_sfp, dsfp0 + static_cast<uint64_t>(((g & 1u) * kSfBytes) >> 4));
+                                if (kVbs && kb == 0) tmem_cp_sf(t_sfv, make_smem_desc(smem_base + SmemLayout::sfv + st * kSfBytes, 0, 128, kSwizzleNone));
                                 const uint32_t id = idesc_pv_bs | (static_cast<uint32_t>(kb) << 29) | (static_cast<uint32_t>(kb) << 4);
                                 mma_mxf8_ts(tmem + kColO, t_p + 8 * kb, dv, id, t_sfp + (static_cast<uint32_t>(kb) << 30), t_sfv + (static_cast<uint32_t>(kb) << 30),
                                             (i > 0 || kb > 0) ? 1u : 0u);
@@ -747,10 +769,29 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             out = __uint_as_float(o.x);
             return true;
         };
-        // the reference the row has after tile g, published by the thread that handled it
-        auto ref_slot = [&](uint32_t g) { return xref + 8u * ((g & 3u) * 128u + r); };
+        // what tile g did to the row's reference, published by the thread that handled it
+        auto ref_slot = [&](uint32_t g) { return xref + 8u * ((g & 7u) * 128u + r); };
 
+        // P of a tile is handed over under the next tile's tensor-memory round trip (or when the role ends): the wait for its stores is then free
+        bool p_ready = false;
+        auto hand_over_p = [&]() {
+            if (!p_ready) return;
+            tmem_wait_st();
+            tc_fence_before_sync();
+            mbar_arrive(bar_p_full(par));
+            p_ready = false;
+        };
         const bool want_fin = kSplit || p.lse_nat != nullptr || cta_traced || kPair;   // does anything read the final reference?
+        float sf_held = 0.0f;   // log2 of the four block scales this group's buffer holds for the row, if they are equal
+        auto scale_o = [&](float f) {
+#pragma unroll 1
+            for (int c = 0; c < 2; ++c) scale_tmem64(t_o_part + 64 * c, f);
+            uint32_t lv;   // the row sum lives in column 0 of L
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(lv) : "r"(t_l) : "memory");
+            tmem_wait_ld();
+            lv = __float_as_uint(__uint_as_float(lv) * f);
+            asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(t_l), "r"(lv) : "memory");
+        };
         uint32_t g0 = 0, n = 0;   // tile counter at the item's first tile; ordinal of the item
         for (uint32_t w = blockIdx.x; ok && w < n_items; w += stride, ++n) {
             // the tile count, the number of tiles every row sees in full and the row's own key limit stay live through the tile loop
@@ -769,14 +810,30 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             const bool tracing = cta_traced && n == 0;
             const bool dumping = tracing && !(p.flags & 0x4u);   // flag 0x4: time stamps only, no tile dumps
             float ref = -INFINITY;   // the row's reference (log2 units) after the last tile this thread has seen
+            float base = -INFINITY;  // long-sequence recipe: what the row's O and L are in units of
 
-            // The tile body exists twice: the copy in the loop has no code for keys past the range; an item's ragged last tile, if this parity
-            // owns it, runs through a second copy placed behind the loop (with all SMs busy, instruction fetch is scarce enough that even
-            // never-executed masking code inside the loop costs 3-4 %; moving the rare rescale out of the loop the same way did not pay).
-            auto tile = [&](int j, auto masked_c) {
-                uint32_t v[128];   // the row's scores, converted in place below
-                float f = 1.0f;    // factor of a rescale
-                bool pv_seen = false;   // P V of this parity's previous tile is known to be done
+            uint32_t v[128];         // the row's scores of a tile, converted in place
+            uint32_t pw[kCols / 4];  // the row's P words
+            auto chunk = [&](int ch) -> uint32_t(&)[32] { return *reinterpret_cast<uint32_t(*)[32]>(&v[32 * ch]); };
+            auto mask_scores = [&](int j) {   // keys past the range: -inf for the maximum, 0 for P (crates/amdgpu-tile/src/reduce.rs:35-49)
+                const int valid = row_lim - j * kKeys;   // may be <= 0 on the causal diagonal: the row then has no key in this tile
+#pragma unroll
+                for (int c = 0; c < 128; ++c) {
+                    if (c >= valid) v[c] = 0xFF800000u;
+                }
+            };
+
+            // ---- the long-sequence recipe
+            // Every block of 32 keys has a reference of its own: P = 2^(s - ref + offset) in e4m3, and its P V goes into O with the block scale
+            // 2^(ref - base) on P (one E8M0 per row and 32 keys of the A operand); base is the row's reference after its first tile. So O is not rescaled
+            // when a row's maximum grows, and no group waits for the other one's reference. O and the row sums are in units of
+            // 2^(base - offset), in f32; only a row that grows by more than kRebase binades past its base (f32 has room for twice that) gets a
+            // new base, and O and L are then rescaled in tensor memory.
+            // A block's reference is the one before it (of this group's last tile, or of the other group's tile before that if that is higher), or
+            // ceil(block maximum) if the maximum passes that by more than the threshold: an integer that only grows within an item.
+            // The maximum of block b + 1 is taken while block b is converted. The conversion is a software pipeline over the 32 words: word c's
+            // exp2 (two values) and bit-built values (two) are started kConvDepth words before they are packed.
+            auto tile_lazy = [&](int j, auto masked_c) {
                 constexpr bool kMasked = decltype(masked_c)::value;
                 const uint32_t g = g0 + static_cast<uint32_t>(j);
                 const uint32_t k = g >> 1;   // this parity's tile counter
@@ -785,21 +842,147 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 if (!mbar_wait(bar_s_full(par), k & 1u, abort_flag)) ok = false;   // no divergent exit: a failed wait only clears `ok`, the vote after the tile loop ends the role
                 tc_fence_after_sync();
                 stamp(st_trace, par, static_cast<int>(g), 1);
-                // All 128 scores of the row in registers with one tensor-memory round trip; the score buffer is handed back at once, so
-                // that Q K^T of tile g + 2 runs under this tile's conversion. The scores are converted in place further down.
-#pragma unroll
-                for (int ch = 0; ch < 4; ++ch) tmem_ld32(t_s + 32 * ch, *reinterpret_cast<uint32_t(*)[32]>(&v[32 * ch]));
-                pv_seen = k == 0 || mbar_test_wait(bar_o_done(par), (k - 1u) & 1u);   // probed under the tensor-memory round trip
+                tmem_ld32(t_s, chunk(0));
+                hand_over_p();
                 tmem_wait_ld();
+                reg_fence32(chunk(0));
+#pragma unroll
+                for (int ch = 1; ch < 4; ++ch) tmem_ld32(t_s + 32 * ch, chunk(ch));
+                if (kMasked) {
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int ch = 1; ch < 4; ++ch) reg_fence32(chunk(ch));
+                    mask_scores(j);
+                }
+                float m[4] = {}, refs[4], sh = 0.0f, cf = 0.0f;
+                auto max_words = [&](int c) {   // two words, four independent chains
+                    m[0] = max3(m[0], __uint_as_float(v[4 * c]), __uint_as_float(v[4 * c + 1]));
+                    m[1] = max3(m[1], __uint_as_float(v[4 * c + 2]), __uint_as_float(v[4 * c + 3]));
+                    m[2] = max3(m[2], __uint_as_float(v[4 * c + 4]), __uint_as_float(v[4 * c + 5]));
+                    m[3] = max3(m[3], __uint_as_float(v[4 * c + 6]), __uint_as_float(v[4 * c + 7]));
+                };
+                auto max_reset = [&]() { m[0] = m[1] = m[2] = m[3] = -INFINITY; };
+                auto next_reference = [&](int b) {
+                    const float mt = fmaxf(max3(m[0], m[1], m[2]), m[3]);
+                    if (mt - kLazyThreshold > ref) ref = ceilf(mt);
+                    refs[b] = ref;
+                };
+                auto use_reference = [&](int b) {
+                    const float x = kMasked && refs[b] == -INFINITY ? 0.0f : refs[b];   // no key in sight yet (causal diagonal): every P is 0 whatever the reference
+                    sh = kPOffset - x;
+                    cf = (kPOffset + 7.0f - kFastBias - x) * 0x1p-21f;
+                };
+                constexpr int kConvDepth = 8;
+                auto conv_start = [&](int c) {
+                    add2(v[4 * c], v[4 * c + 1], sh);
+                    v[4 * c] = __float_as_uint(ex2_approx(__uint_as_float(v[4 * c])));
+                    v[4 * c + 1] = __float_as_uint(ex2_approx(__uint_as_float(v[4 * c + 1])));
+                    fma2(v[4 * c + 2], v[4 * c + 3], 0x1p-21f, cf);
+                };
+                auto conv_finish = [&](int d) {
+                    const uint32_t lo = cvt_e4m3x2(__uint_as_float(v[4 * d]), __uint_as_float(v[4 * d + 1]));
+                    pw[d] = __byte_perm(lo, cvt_relu_f16x2(__uint_as_float(v[4 * d + 2]), __uint_as_float(v[4 * d + 3])), 0x6410);
+                };
+                if (dumping && j == 0) {
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int c = 0; c < 128; ++c) p.trace[r * 128 + c] = __uint_as_float(v[c]);
+                }
+                max_reset();
+#pragma unroll
+                for (int c = 0; c < 8; c += 2) max_words(c);
+                next_reference(0);
+                use_reference(0);
+                if (!kMasked) {
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int ch = 1; ch < 4; ++ch) reg_fence32(chunk(ch));
+                }
+                // the scores are in registers: Q K^T of tile g + 2 may overwrite them
                 tc_fence_before_sync();
                 mbar_arrive(bar_s_free(par));
-                if (kMasked) {   // keys past the range: -inf for the maximum, 0 for P (crates/amdgpu-tile/src/reduce.rs:35-49)
-                    const int valid = row_lim - j * kKeys;   // may be <= 0 on the causal diagonal: the row then has no key in this tile
+                stamp(st_trace, par, static_cast<int>(g), 2);
+                bool pv_seen = false;
+                uint2 prev = make_uint2(0u, g);   // (tag g: not the one looked for)
 #pragma unroll
-                    for (int c = 0; c < 128; ++c) {
-                        if (c >= valid) v[c] = 0xFF800000u;
+                for (int c = 0; c < 32 + kConvDepth; ++c) {
+                    if (c % 8 == 0 && c > 0 && c < 32) use_reference(c / 8);
+                    if (c < 32) conv_start(c);
+                    if (c < 24) {
+                        if (c % 8 == 0) max_reset();
+                        if (c % 2 == 0) max_words(c + 8);
+                        if (c % 8 == 7) next_reference(c / 8 + 1);
+                    }
+                    if (c == 24) {
+                        st_shared_v2(ref_slot(g), __float_as_uint(ref), g);
+                        pv_seen = k == 0 || mbar_test_wait(bar_o_done(par), (k - 1u) & 1u);   // probed ahead: P V of this parity's previous tile
+                    }
+                    if (c == 32 && j > 0) prev = ld_shared_v2(ref_slot(g - 1u));
+                    if (c >= kConvDepth) conv_finish(c - kConvDepth);
+                }
+                if (dumping && j == 0) {
+#pragma unroll
+                    for (int c = 0; c < kCols / 4; ++c) reinterpret_cast<uint32_t*>(p.trace)[32768 + 256 + r * 32 + c] = pw[c];
+                }
+                stamp(st_trace, par, static_cast<int>(g), 5);
+                // The row's base after the previous tile and after this one. Both groups follow the published references with the same rule, so
+                // they agree on it; the reference of the previous tile was published a tile's time ago
+                float ref_prev = __uint_as_float(prev.x), base_prev = base;
+                if (j > 0) {
+                    if (prev.y != g - 1u && ok && !wait_slot(ref_slot(g - 1u), g - 1u, ref_prev)) ok = false;
+                    if (ref_prev - base > kRebase) base_prev = ref_prev;
+                } else {
+                    base_prev = ref;
+                }
+                base = ref - base_prev > kRebase ? ref : base_prev;
+                const bool rebase = base != base_prev;
+                // P V of this parity's previous tile must be done before its P columns and scales are overwritten (and, observed in order,
+                // this keeps the phase parity of the other parity's barrier below unambiguous)
+                if (!pv_seen && !mbar_wait(bar_o_done(par), (k - 1u) & 1u, abort_flag)) ok = false;
+                // The item's last tile leaves the row's base for the epilogue warpgroup's log-sum-exp: before this thread's arrive
+                // on p_full (which the last P V, and through it the epilogue's o_full, come after), and behind the wait above: P V of tile
+                // g - 2 is done, so P V of g - 3 is, so the epilogue has taken the item four back out (o_free) and read its slot
+                if (want_fin && j == n_tiles - 1) *reinterpret_cast<volatile float*>(smem_gen + SmemLayout::xfin + 4u * ((n & 3u) * 128u + r)) = base;
+                stamp(st_trace, par, static_cast<int>(g), 6);
+                tmem_st32(t_p, pw);
+                // the row's four scale bytes (one per 32 keys), in the pattern that tcgen05.cp spreads over the lane quadrants; they rarely change
+                const float above = refs[0] - base;
+                if (__builtin_expect(__any_sync(0xFFFFFFFFu, above != sf_held || ref != refs[0] || rebase), 0)) {
+                    uint32_t sf[4];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) sf[b] = __float_as_uint(fmaxf(refs[b] - base, -127.0f) + 8388735.0f);   // E8M0 in the low byte: exponent + 127
+                    reinterpret_cast<volatile uint32_t*>(smem_gen + SmemLayout::sfp + par * kSfBytes)[(r & 31u) * 4u + (r >> 5)] =
+                        __byte_perm(__byte_perm(sf[0], sf[1], 0x0040), __byte_perm(sf[2], sf[3], 0x0040), 0x5410);
+                    sf_held = ref == refs[0] ? above : INFINITY;   // four equal scales, or to be written again
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (j > 0 && __any_sync(0xFFFFFFFFu, rebase)) {
+                        if (!mbar_wait(bar_o_done(par ^ 1u), ((g - 1u) >> 1) & 1u, abort_flag)) ok = false;
+                        __syncwarp();
+                        tc_fence_after_sync();
+                        scale_o(rebase ? ex2_approx(base_prev - base) : 1.0f);
                     }
                 }
+                if (j > 0) ref = fmaxf(ref, ref_prev);
+                p_ready = true;
+                stamp(st_trace, par, static_cast<int>(g), 7);
+            };
+
+            // ---- the short-sequence recipe: the reference follows every tile's maximum (within a window), O and L are rescaled when it moves
+            auto tile_short = [&](int j, bool masked) {
+                const uint32_t g = g0 + static_cast<uint32_t>(j);
+                const uint32_t k = g >> 1;
+                if (!mbar_wait(bar_s_full(par), k & 1u, abort_flag)) ok = false;
+                tc_fence_after_sync();
+#pragma unroll
+                for (int ch = 0; ch < 4; ++ch) tmem_ld32(t_s + 32 * ch, chunk(ch));
+                hand_over_p();
+                tmem_wait_ld();
+#pragma unroll
+                for (int ch = 0; ch < 4; ++ch) reg_fence32(chunk(ch));
+                if (masked) mask_scores(j);
+                tc_fence_before_sync();
+                mbar_arrive(bar_s_free(par));
                 if (dumping && j == 0) {
 #pragma unroll
                     for (int c = 0; c < 128; ++c) p.trace[r * 128 + c] = __uint_as_float(v[c]);
@@ -808,101 +991,48 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
                 for (int i = 0; i < 8; ++i) m[i] = -INFINITY;
 #pragma unroll
-                for (int c = 0; c < 128; c += 16) {   // eight independent chains of three-input maxima
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) m[i] = max3(m[i], __uint_as_float(v[c + 2 * i]), __uint_as_float(v[c + 2 * i + 1]));
-                }
+                for (int c = 0; c < 128; c += 2) m[(c / 2) & 7] = max3(m[(c / 2) & 7], __uint_as_float(v[c]), __uint_as_float(v[c + 1]));
                 const float mt = fmaxf(fmaxf(max3(m[0], m[1], m[2]), max3(m[3], m[4], m[5])), fmaxf(m[6], m[7]));
-                stamp(st_trace, par, static_cast<int>(g), 2);
-                stamp(st_trace, par, static_cast<int>(g), 3);
-                // The hand-over of the row's reference from the thread that handled the item's previous tile is the one dependency that runs
-                // from tile to tile across the two groups, so everything that does not need the old reference is computed before the slot is
-                // read, and the new reference is published before the rescale factor is worked out.
-                const float cand = lazy ? ceilf(mt) : mt;   // where the reference goes if it moves
-                const float mt_thr = mt - thr;
                 if (ok && j > 0 && !wait_slot(ref_slot(g - 1u), g - 1u, ref)) ok = false;
-                // the reference moves when this tile's maximum passes it by more than the threshold (negative for short sequences: it then
-                // also follows the tile maximum down, and f > 1 scales O and L up)
-                const bool move = mt_thr > ref;
-                const float old_ref = ref;
-                ref = move ? cand : ref;
+                // moves when the tile maximum lies above the reference or less than the window below it: f > 1 scales O and L up
+                const bool move = mt + kFollowWindow > ref;
+                const float f = move ? ex2_approx(ref - mt) : 1.0f;   // 0 on the first tile (old reference -inf)
+                ref = move ? mt : ref;
                 st_shared_v2(ref_slot(g), __float_as_uint(ref), g);
-                f = move ? ex2_approx(old_ref - ref) : 1.0f;   // 0 on the first tile (old reference -inf); an exact power of two for integer references
-                stamp(st_trace, par, static_cast<int>(g), 4);
-                // P V of this parity's previous tile must be done before its P columns are overwritten (and, observed in order, this keeps
-                // the phase parity of the other parity's barrier below unambiguous)
-                if (!pv_seen && k > 0 && !mbar_wait(bar_o_done(par), (k - 1u) & 1u, abort_flag)) ok = false;
-                stamp(st_trace, par, static_cast<int>(g), 5);
-                // The item's last tile leaves the row's final reference for the epilogue warpgroup's log-sum-exp: before this thread's arrive
-                // on p_full (which the last P V, and through it the epilogue's o_full, come after), and behind the wait above: P V of tile
-                // g - 2 is done, so P V of g - 3 is, so the epilogue has taken the item four back out (o_free) and read its slot
+                if (k > 0 && !mbar_wait(bar_o_done(par), (k - 1u) & 1u, abort_flag)) ok = false;
                 if (want_fin && j == n_tiles - 1) *reinterpret_cast<volatile float*>(smem_gen + SmemLayout::xfin + 4u * ((n & 3u) * 128u + r)) = ref;
-                if (__builtin_expect(j > 0 && __any_sync(0xFFFFFFFFu, move), 0)) {
-                    // O holds P V of all the item's tiles before j once the other parity's last P V is done; P V of tile j cannot start before this thread's arrive below
-                    if (!mbar_wait(bar_o_done(par ^ 1u), ((g - 1u) >> 1) & 1u, abort_flag)) ok = false;
-                    tc_fence_after_sync();
-    #pragma unroll 1
-                    for (int c = 0; c < kCols / 32; ++c) scale_tmem32(t_o_part + 32 * c, f);
-                    {   // the row sum lives in column 0 of L
-                        uint32_t lv;
-                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(lv) : "r"(t_l) : "memory");
-                        tmem_wait_ld();
-                        lv = __float_as_uint(__uint_as_float(lv) * f);
-                        asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(t_l), "r"(lv) : "memory");
-                    }
-                    tmem_wait_st();
-                }
-                // P = e4m3(2^(s - ref + offset)), four keys per 32-bit TMEM column
-                const float sh = kPOffset - ref;
-                const float cf = (kPOffset + 7.0f - kFastBias - ref) * 0.03125f;
-                uint32_t pw[kCols / 4];
-                if (lazy) {
-                    // Software pipeline over the 32 words, in place in the score registers: word c's exp2 (two values) and bit-built values
-                    // (two) are started kConvDepth words before they are converted and packed, so that a thread always has that many
-                    // independent chains in flight without holding more than the score row itself (+2 % on the headline shape over one word
-                    // at a time; depths 4, 16 and 32 and scheduling points between the words were slower).
-                    constexpr int kConvDepth = 8;
+                const float s0 = kPOffset - ref;
 #pragma unroll
-                    for (int c = 0; c < 32 + kConvDepth; ++c) {
-                        if (c < 32) {
-                            add2(v[4 * c], v[4 * c + 1], sh);
-                            v[4 * c] = __float_as_uint(ex2_approx(__uint_as_float(v[4 * c])));
-                            v[4 * c + 1] = __float_as_uint(ex2_approx(__uint_as_float(v[4 * c + 1])));
-                            v[4 * c + 2] = fast_p_sat(v[4 * c + 2], cf);
-                            v[4 * c + 3] = fast_p_sat(v[4 * c + 3], cf);
-                            add2(v[4 * c + 2], v[4 * c + 3], 32768.0f);
-                        }
-                        if (c >= kConvDepth) {
-                            const int d = c - kConvDepth;
-                            const uint32_t lo = cvt_e4m3x2(__uint_as_float(v[4 * d]), __uint_as_float(v[4 * d + 1]));
-                            const uint32_t hi = __byte_perm(v[4 * d + 2], v[4 * d + 3], 0x0040);
-                            pw[d] = __byte_perm(lo, hi, 0x5410);
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) pw[c] = p_word(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3], sh);
-                }
+                for (int c = 0; c < 32; ++c) pw[c] = p_word(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3], s0);
                 if (dumping && j == 0) {
 #pragma unroll
                     for (int c = 0; c < kCols / 4; ++c) reinterpret_cast<uint32_t*>(p.trace)[32768 + 256 + r * 32 + c] = pw[c];
                 }
-                stamp(st_trace, par, static_cast<int>(g), 6);
                 tmem_st32(t_p, pw);
-                tmem_wait_st();
-                tc_fence_before_sync();
-                mbar_arrive(bar_p_full(par));
-                stamp(st_trace, par, static_cast<int>(g), 7);
+                if (j > 0 && __any_sync(0xFFFFFFFFu, move)) {
+                    // O holds P V of all the item's tiles before j once the other parity's last P V is done; P V of tile j cannot start before P is handed over
+                    if (!mbar_wait(bar_o_done(par ^ 1u), ((g - 1u) >> 1) & 1u, abort_flag)) ok = false;
+                    __syncwarp();
+                    tc_fence_after_sync();
+                    scale_o(f);
+                }
+                p_ready = true;
             };
             // tiles [0, j_full) have all their keys for every row; behind them come at most two tiles (a ragged end: one; the causal
             // diagonal: up to two), of which this parity owns at most one
             int j = static_cast<int>((g0 ^ par) & 1u);
-            for (; j < j_full; j += 2) tile(j, std::false_type{});
-            if (j < n_tiles) tile(j, std::true_type{});
+            if constexpr (lazy) {
+                // the loop has no code for keys past the range: with all SMs busy instruction fetch is scarce enough that it would cost 3 %
+                for (; j < j_full; j += 2) tile_lazy(j, std::false_type{});
+                if (j < n_tiles) tile_lazy(j, std::true_type{});
+            } else {
+                for (; j < n_tiles; j += 2) tile_short(j, j >= j_full);
+            }
             // a failed wait above only clears `ok`; the warp leaves as one
             if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
             g0 += static_cast<uint32_t>(n_tiles);
         }
+        hand_over_p();
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kEpilogueRegs));
         // =========================================================== epilogue ===========================================================

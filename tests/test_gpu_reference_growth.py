@@ -1,0 +1,51 @@
+"""Rows whose maximum grows, falls or jumps along the keys: the block scales on P, and the new base of a row that grows by more binades than they are
+let cover, against the fp64 oracle and the reference path on the same inputs."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+# exponent added to the K scales of key tile t of n: the scores of the tile grow by 2^that, from a few binades to a few hundred
+PATTERNS = {
+    "slow": lambda t, n: t * 3 // n,
+    "up": lambda t, n: t * 7 // n,
+    "down": lambda t, n: (n - 1 - t) * 7 // n,
+    "jump": lambda t, n: 7 if t == n // 2 else 0,
+    "jump_odd_last": lambda t, n: 7 if t == n - 1 else 0,
+    "alternate": lambda t, n: 6 * (t & 1),
+}
+
+
+@pytest.mark.parametrize("pattern", PATTERNS)
+@pytest.mark.parametrize("shape,path,splits", [((1, 2, 200, 1337, 2), "vs128", None), ((2, 2, 256, 512, 1), "t128", None), ((1, 2, 256, 2100, 2), "kvsplit", 4),
+                                               ((1, 1, 256, 16384, 1), "vs128", None)], ids=lambda s: str(s).replace(" ", ""))
+def test_growing_rows(oracle, pattern, shape, path, splits):
+    from amdgpu_rustdsl_b200 import device_status, fmha_fwd_mxfp8
+    B, H, S, SK, g = shape
+    HK = H // g
+    inp = oracle.generate("normal", B, H, S, SK, HK)
+    n = -(-SK // 128)
+    add = np.repeat([PATTERNS[pattern](t, n) for t in range(n)], 128)[:SK].astype(np.uint8)
+    ks = inp.ks.copy()
+    ks[: B * SK * HK * 4].reshape(B, SK, HK, 4)[...] += add[None, :, None, None]
+    inp = oracle.Inputs(B, H, HK, S, SK, inp.q, inp.k, inp.v, inp.qs, ks, inp.vdescale)
+    q, k, v, qs, kd = (torch.from_numpy(x).cuda() for x in (inp.q, inp.k, inp.v, inp.qs, ks))
+    vs = torch.zeros(1024, dtype=torch.float32, device="cuda")
+    vs[0] = inp.vdescale
+    out = torch.full((B, S, H, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    fmha_fwd_mxfp8(q, k, v, qs, kd, vs, out, path=path, splits=splits)
+    torch.cuda.synchronize()
+    got = out.view(torch.int16).cpu().numpy().view(np.uint16)
+    rows = list(range(S))
+    ref = oracle.reference(inp, rows)
+    ours = oracle.compare(inp, got, ref, rows)
+    theirs = oracle.compare(inp, oracle.recipe_forward(inp, rows, 0), ref, rows)
+    # A weight of P is off by 2^-4 at most from e4m3 rounding and 0.062 from the linear mantissa, in the sum as in the product: with weights
+    # w(1 + d), |d| <= 0.125, an output moves by at most 2 * 0.125 / (1 - 0.125) of the largest |v| of its column
+    bound = 0.29 * float(np.abs(oracle.e4m3_table()[inp.v]).max()) * inp.vdescale
+    assert ours.worst_err <= bound, (ours, theirs)
+    # The gate's 1.10 on the mean, and two standard errors of it: a few keys carry such a row, so its 128 errors are one or two roundings of P, and
+    # with 200 rows whose errors spread by 1 to 1.5 of their mean the ratio of two means is uncertain by sqrt(2) * 1 / sqrt(200) = 0.1 or so
+    assert ours.mean_err <= (1.10 + 0.2) * theirs.mean_err, (ours, theirs)
+    assert device_status() == 0
