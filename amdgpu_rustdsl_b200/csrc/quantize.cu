@@ -10,7 +10,10 @@
 // bit for bit. Inputs must be finite. Both kernels are pure streaming: 2 bytes in, 1 (+ 1/32) byte out per element.
 #include "kernels.h"
 
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 namespace b200mx {
 
@@ -22,112 +25,258 @@ __device__ __forceinline__ uint32_t e4m3x2(float lo, float hi) {
     return h;
 }
 
-// One thread = 8 consecutive elements (16 bytes in, 8 bytes out); 4 threads = one 32-element block; 16 threads = one row of 128.
+// Programmatic dependent launch, both sides: the launch behind this one may be scheduled while this grid runs, and nothing above the wait touches
+// global memory. A short prompt's chain (Q, K, V, attention) is launches more than work.
+__device__ __forceinline__ void pdl_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// A 16-byte read-once load. Volatile, so that it stays behind the wait above (a plain __ldg is an invariant load, which may move across it).
+__device__ __forceinline__ uint4 ld_vec(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+// 8 consecutive elements (16 bytes in, 8 bytes out) of one 32-element block per lane; 4 lanes = one block, 16 lanes = one row of 128. All 32 lanes
+// take part (shuffles); a lane that is not live has zeros and stores nothing.
+__device__ __forceinline__ void quantize_qk_vec(const uint4 raw, bool live, float mul, unsigned lane, unsigned long long t, uint2* __restrict__ out, uint32_t* __restrict__ scales) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+    float y[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        y[2 * i] = __fmul_rn(__uint_as_float(w[i] << 16), mul);
+        y[2 * i + 1] = __fmul_rn(__uint_as_float(w[i] & 0xFFFF0000u), mul);
+    }
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(y[i]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+    // floor(log2 amax) of a normal f32 is its exponent field - 127; zero and subnormal maxima end at the lower clamp either way
+    int eb = static_cast<int>((__float_as_uint(amax) >> 23) & 0xFFu) - 8;
+    eb = eb < 0 ? 0 : (eb > 254 ? 254 : eb);
+    // x * 2^(127 - eb) as two exact multiplications by normal powers of two (the exponent 127 - eb lies in [-127, 127]; a value that
+    // an intermediate product flushes or rounds is far below the smallest e4m3 step in the end and encodes as zero either way)
+    const int sh = 127 - eb, sh1 = sh >> 1, sh2 = sh - sh1;
+    const float s1 = __uint_as_float(static_cast<uint32_t>(127 + sh1) << 23), s2 = __uint_as_float(static_cast<uint32_t>(127 + sh2) << 23);
+    uint32_t b[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        b[i] = e4m3x2(__fmul_rn(__fmul_rn(y[4 * i], s1), s2), __fmul_rn(__fmul_rn(y[4 * i + 1], s1), s2)) |
+               (e4m3x2(__fmul_rn(__fmul_rn(y[4 * i + 2], s1), s2), __fmul_rn(__fmul_rn(y[4 * i + 3], s1), s2)) << 16);
+    }
+    if (live) out[t] = make_uint2(b[0], b[1]);
+    // the row's four scale bytes: lanes 0, 4, 8, 12 of each 16-lane half hold them
+    const uint32_t e1 = __shfl_down_sync(0xFFFFFFFFu, static_cast<uint32_t>(eb), 4);
+    const uint32_t e2 = __shfl_down_sync(0xFFFFFFFFu, static_cast<uint32_t>(eb), 8);
+    const uint32_t e3 = __shfl_down_sync(0xFFFFFFFFu, static_cast<uint32_t>(eb), 12);
+    if (live && (lane & 15u) == 0u) scales[t >> 4] = static_cast<uint32_t>(eb) | (e1 << 8) | (e2 << 16) | (e3 << 24);
+}
+
+// kVecs 16-byte loads of a thread are in flight before the first is used: bound by DRAM, and one load per thread at a time does not cover its latency.
+template <int kVecs>
 __global__ void __launch_bounds__(256) quantize_qk_kernel(const uint4* __restrict__ x, unsigned long long rows, float mul,
                                                           uint2* __restrict__ out, uint32_t* __restrict__ scales) {
-    const unsigned long long n_threads = rows * 16ull;
+    pdl_begin();
+    const unsigned long long n_threads = rows * 16ull, step = static_cast<unsigned long long>(gridDim.x) * (256u * kVecs);
     const unsigned lane = threadIdx.x & 31u;
-    for (unsigned long long t0 = (static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x) & ~31ull; t0 < n_threads;
-         t0 += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
-        const unsigned long long t = t0 + lane;   // whole warps stay in the loop together: the shuffles below need all lanes
-        const bool live = t < n_threads;
-        float y[8];
-        if (live) {
-            const uint4 raw = __ldg(x + t);
-            const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+    // t0: the warp's first vector; whole warps stay in the loop together: the shuffles need all lanes
+    for (unsigned long long t0 = static_cast<unsigned long long>(blockIdx.x) * (256u * kVecs) + (threadIdx.x & ~31u); t0 < n_threads; t0 += step) {
+        uint4 raw[kVecs];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                y[2 * i] = __fmul_rn(__uint_as_float(w[i] << 16), mul);
-                y[2 * i + 1] = __fmul_rn(__uint_as_float(w[i] & 0xFFFF0000u), mul);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) y[i] = 0.0f;
+        for (int i = 0; i < kVecs; ++i) {
+            const unsigned long long t = t0 + lane + 256u * i;
+            raw[i] = t < n_threads ? ld_vec(x + t) : make_uint4(0u, 0u, 0u, 0u);
         }
-        float amax = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(y[i]));
-        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
-        // floor(log2 amax) of a normal f32 is its exponent field - 127; zero and subnormal maxima end at the lower clamp either way
-        int eb = static_cast<int>((__float_as_uint(amax) >> 23) & 0xFFu) - 8;
-        eb = eb < 0 ? 0 : (eb > 254 ? 254 : eb);
-        // x * 2^(127 - eb) as two exact multiplications by normal powers of two (the exponent 127 - eb lies in [-127, 127]; a value that
-        // an intermediate product flushes or rounds is far below the smallest e4m3 step in the end and encodes as zero either way)
-        const int sh = 127 - eb, sh1 = sh >> 1, sh2 = sh - sh1;
-        const float s1 = __uint_as_float(static_cast<uint32_t>(127 + sh1) << 23), s2 = __uint_as_float(static_cast<uint32_t>(127 + sh2) << 23);
-        uint32_t b[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            b[i] = e4m3x2(__fmul_rn(__fmul_rn(y[4 * i], s1), s2), __fmul_rn(__fmul_rn(y[4 * i + 1], s1), s2)) |
-                   (e4m3x2(__fmul_rn(__fmul_rn(y[4 * i + 2], s1), s2), __fmul_rn(__fmul_rn(y[4 * i + 3], s1), s2)) << 16);
+        for (int i = 0; i < kVecs; ++i) {
+            const unsigned long long t = t0 + lane + 256u * i;
+            quantize_qk_vec(raw[i], t < n_threads, mul, lane, t, out, scales);
         }
-        if (live) out[t] = make_uint2(b[0], b[1]);
-        // the row's four scale bytes: lanes 0, 4, 8, 12 of each 16-lane half hold them
-        const uint32_t e1 = __shfl_down_sync(0xFFFFFFFFu, static_cast<uint32_t>(eb), 4);
-        const uint32_t e2 = __shfl_down_sync(0xFFFFFFFFu, static_cast<uint32_t>(eb), 8);
-        const uint32_t e3 = __shfl_down_sync(0xFFFFFFFFu, static_cast<uint32_t>(eb), 12);
-        if (live && (lane & 15u) == 0u) scales[t >> 4] = static_cast<uint32_t>(eb) | (e1 << 8) | (e2 << 16) | (e3 << 24);
     }
 }
 
-__global__ void __launch_bounds__(256) amax_kernel(const uint4* __restrict__ x, unsigned long long n_vec, uint32_t* __restrict__ amax_bits) {
-    float amax = 0.0f;
-    for (unsigned long long t = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x; t < n_vec;
-         t += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
-        const uint4 raw = __ldg(x + t);
-        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+__device__ __forceinline__ float amax_vec(float amax, const uint4 raw) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(w[i] << 16)), fabsf(__uint_as_float(w[i] & 0xFFFF0000u))));
-    }
+    for (int i = 0; i < 4; ++i) amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(w[i] << 16)), fabsf(__uint_as_float(w[i] & 0xFFFF0000u))));
+    return amax;
+}
+
+__device__ __forceinline__ float amax_warp(float amax) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-    if ((threadIdx.x & 31u) == 0u) atomicMax(amax_bits, __float_as_uint(amax));   // non-negative floats order like their bit patterns
+    return amax;
 }
 
-__global__ void __launch_bounds__(256) quantize_v_kernel(const uint4* __restrict__ x, unsigned long long n_vec, uint2* __restrict__ out,
-                                                         float* __restrict__ descale) {
-    const float amax = __uint_as_float(reinterpret_cast<const uint32_t*>(descale)[1]);
-    const float vd = amax > 0.0f ? __fdiv_rn(amax, 448.0f) : 1.0f;
-    if (blockIdx.x == 0 && threadIdx.x == 0) descale[0] = vd;
-    for (unsigned long long t = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x; t < n_vec;
-         t += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
-        const uint4 raw = __ldg(x + t);
-        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-        uint32_t b[2];
+__device__ __forceinline__ float v_descale_of(float amax) { return amax > 0.0f ? __fdiv_rn(amax, 448.0f) : 1.0f; }
+
+// x / vd rounded to nearest even, from r = 1 / vd rounded to nearest: q = x r is within an ulp, and one residual correction rounds it
+// correctly (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990, theorem 7.2). vd is in
+// [kDivLo, kDivHi]: no residual that matters underflows (|x| <= 448 vd (1 + 2^-23); a quotient under 2^-11 is the byte 0 either way). A division
+// costs a tenth of these three instructions' rate and was what the kernel waited for.
+__device__ __forceinline__ float div_by(float x, float vd, float r) {
+    const float q = __fmul_rn(x, r);
+    return __fmaf_rn(__fmaf_rn(-q, vd, x), r, q);
+}
+constexpr float kDivLo = 0x1p-90f, kDivHi = 0x1p100f;
+
+template <bool kFast>
+__device__ __forceinline__ uint2 quantize_v_vec(const uint4 raw, float vd, float r) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+    auto q = [&](uint32_t bits) { return kFast ? div_by(__uint_as_float(bits), vd, r) : __fdiv_rn(__uint_as_float(bits), vd); };
+    uint32_t b[2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            b[i] = e4m3x2(__fdiv_rn(__uint_as_float(w[2 * i] << 16), vd), __fdiv_rn(__uint_as_float(w[2 * i] & 0xFFFF0000u), vd)) |
-                   (e4m3x2(__fdiv_rn(__uint_as_float(w[2 * i + 1] << 16), vd), __fdiv_rn(__uint_as_float(w[2 * i + 1] & 0xFFFF0000u), vd)) << 16);
-        }
-        out[t] = make_uint2(b[0], b[1]);
+    for (int i = 0; i < 2; ++i) {
+        b[i] = e4m3x2(q(w[2 * i] << 16), q(w[2 * i] & 0xFFFF0000u)) | (e4m3x2(q(w[2 * i + 1] << 16), q(w[2 * i + 1] & 0xFFFF0000u)) << 16);
+    }
+    return make_uint2(b[0], b[1]);
+}
+
+template <int kVecs>
+__global__ void __launch_bounds__(256) amax_kernel(const uint4* __restrict__ x, unsigned long long n_vec, uint32_t* __restrict__ amax_bits) {
+    float amax = 0.0f;
+    const unsigned long long step = static_cast<unsigned long long>(gridDim.x) * (256u * kVecs);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    for (unsigned long long t0 = static_cast<unsigned long long>(blockIdx.x) * (256u * kVecs) + threadIdx.x; t0 < n_vec; t0 += step) {
+        uint4 raw[kVecs];
+#pragma unroll
+        for (int i = 0; i < kVecs; ++i) raw[i] = t0 + 256u * i < n_vec ? ld_vec(x + t0 + 256u * i) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int i = 0; i < kVecs; ++i) amax = amax_vec(amax, raw[i]);
+    }
+    amax = amax_warp(amax);
+    __shared__ float part[8];
+    if ((threadIdx.x & 31u) == 0u) part[threadIdx.x >> 5] = amax;
+    __syncthreads();
+    if (threadIdx.x == 0u) {
+#pragma unroll
+        for (int i = 1; i < 8; ++i) amax = fmaxf(amax, part[i]);
+        atomicMax(amax_bits, __float_as_uint(amax));   // non-negative floats order like their bit patterns
     }
 }
 
-int grid_for(unsigned long long threads) {
+// Walks the vectors from the last to the first: the amax pass before it read them in rising order, so the last ones are still in L2.
+template <int kVecs>
+__global__ void __launch_bounds__(256) quantize_v_kernel(const uint4* __restrict__ x, unsigned long long n_vec, uint2* __restrict__ out,
+                                                         float* __restrict__ descale) {
+    pdl_begin();
+    const float amax = __uint_as_float(reinterpret_cast<const volatile uint32_t*>(descale)[1]);
+    const float vd = v_descale_of(amax);
+    if (blockIdx.x == 0 && threadIdx.x == 0) descale[0] = vd;
+    const unsigned long long step = static_cast<unsigned long long>(gridDim.x) * (256u * kVecs);
+    auto pass = [&](auto fast_c, float r) {
+        constexpr bool kFast = decltype(fast_c)::value;
+        for (unsigned long long t0 = static_cast<unsigned long long>(blockIdx.x) * (256u * kVecs) + threadIdx.x; t0 < n_vec; t0 += step) {
+            uint4 raw[kVecs];
+#pragma unroll
+            for (int i = 0; i < kVecs; ++i) raw[i] = t0 + 256u * i < n_vec ? ld_vec(x + (n_vec - 1u - t0 - 256u * i)) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int i = 0; i < kVecs; ++i) {
+                const uint2 b = quantize_v_vec<kFast>(raw[i], vd, r);
+                if (t0 + 256u * i < n_vec) out[n_vec - 1u - t0 - 256u * i] = b;
+            }
+        }
+    };
+    if (vd >= kDivLo && vd <= kDivHi) pass(std::true_type{}, __frcp_rn(vd));
+    else pass(std::false_type{}, 0.0f);
+}
+
+// A small V in one launch: a cluster of 8 CTAs keeps it in registers between the maximum, exchanged through distributed shared memory, and the
+// quantisation. The general form is three launches (clear, maximum, quantise) and reads V twice.
+constexpr unsigned kSmallCtas = 8, kSmallThreads = 1024, kSmallVecs = 4, kSmallMax = kSmallCtas * kSmallThreads * kSmallVecs;
+__global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThreads)
+quantize_v_small_kernel(const uint4* __restrict__ x, unsigned n_vec, uint2* __restrict__ out, float* __restrict__ descale) {
+    namespace cg = cooperative_groups;
+    pdl_begin();
+    __shared__ float part[kSmallThreads / 32];
+    __shared__ float cta_amax[kSmallCtas];   // [source CTA], written by all of them
+    const cg::cluster_group cluster = cg::this_cluster();
+    const unsigned tid = blockIdx.x * kSmallThreads + threadIdx.x;
+    uint4 raw[kSmallVecs];
+#pragma unroll
+    for (unsigned i = 0; i < kSmallVecs; ++i) {
+        const unsigned t = tid + i * (kSmallCtas * kSmallThreads);
+        raw[i] = t < n_vec ? ld_vec(x + t) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    float amax = 0.0f;
+#pragma unroll
+    for (unsigned i = 0; i < kSmallVecs; ++i) amax = amax_vec(amax, raw[i]);
+    amax = amax_warp(amax);
+    if ((threadIdx.x & 31u) == 0u) part[threadIdx.x >> 5] = amax;
+    __syncthreads();
+    if (threadIdx.x < 32u) {
+        amax = amax_warp(part[threadIdx.x]);
+        if (threadIdx.x < kSmallCtas) *cluster.map_shared_rank(&cta_amax[blockIdx.x], threadIdx.x) = amax;
+    }
+    cluster.sync();   // (nobody touches another CTA's shared memory behind it)
+    amax = cta_amax[0];
+#pragma unroll
+    for (unsigned i = 1; i < kSmallCtas; ++i) amax = fmaxf(amax, cta_amax[i]);
+    const float vd = v_descale_of(amax);
+    if (tid == 0u) {
+        descale[0] = vd;
+        reinterpret_cast<uint32_t*>(descale)[1] = __float_as_uint(amax);   // what the general form leaves there
+    }
+    const bool fast = vd >= kDivLo && vd <= kDivHi;
+    const float r = fast ? __frcp_rn(vd) : 0.0f;
+#pragma unroll
+    for (unsigned i = 0; i < kSmallVecs; ++i) {
+        const unsigned t = tid + i * (kSmallCtas * kSmallThreads);
+        if (t < n_vec) out[t] = fast ? quantize_v_vec<true>(raw[i], vd, r) : quantize_v_vec<false>(raw[i], vd, r);
+    }
+}
+
+// Blocks of 256 threads with `vecs` vectors each; grid-stride beyond 8 CTAs per SM
+int grid_for(unsigned long long n_vec, unsigned vecs) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const unsigned long long blocks = (threads + 255) / 256, cap = 8ull * static_cast<unsigned long long>(sms);   // grid-stride beyond 8 CTAs per SM
+    const unsigned long long blocks = (n_vec + 256u * vecs - 1) / (256u * vecs), cap = 8ull * static_cast<unsigned long long>(sms);
     return static_cast<int>(blocks < cap ? (blocks ? blocks : 1) : cap);
 }
+
+template <typename... Params, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(Params...), unsigned grid, unsigned threads, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+// From 4 vectors per thread of a full machine on: the wide form then still has every SM's thread slots filled.
+constexpr unsigned long long kWideVecs = 4ull * 148ull * 2048ull;
 
 }  // namespace
 
 cudaError_t launch_quantize_qk(const void* x_bf16, unsigned long long rows, float mul, void* out_e4m3, void* out_scales, cudaStream_t stream) {
-    quantize_qk_kernel<<<grid_for(rows * 16ull), 256, 0, stream>>>(static_cast<const uint4*>(x_bf16), rows, mul, static_cast<uint2*>(out_e4m3),
-                                                                   static_cast<uint32_t*>(out_scales));
-    return cudaGetLastError();
+    const unsigned long long n_vec = rows * 16ull;
+    const bool wide = n_vec >= kWideVecs;
+    return launch_pdl(wide ? quantize_qk_kernel<4> : quantize_qk_kernel<1>, grid_for(n_vec, wide ? 4u : 1u), 256u, stream, static_cast<const uint4*>(x_bf16), rows, mul,
+                      static_cast<uint2*>(out_e4m3), static_cast<uint32_t*>(out_scales));
 }
 
 cudaError_t launch_quantize_v(const void* x_bf16, unsigned long long n_elems, void* out_e4m3, float* descale, cudaStream_t stream) {
+    const unsigned long long n_vec = n_elems / 8;
+    const uint4* x = static_cast<const uint4*>(x_bf16);
+    uint2* out = static_cast<uint2*>(out_e4m3);
+    if (n_vec <= kSmallMax) return launch_pdl(quantize_v_small_kernel, kSmallCtas, kSmallThreads, stream, x, static_cast<unsigned>(n_vec), out, descale);
     cudaError_t e = cudaMemsetAsync(descale, 0, 8, stream);   // [0] the descale, [1] the running maximum's bits
     if (e != cudaSuccess) return e;
-    const unsigned long long n_vec = n_elems / 8;
-    amax_kernel<<<grid_for(n_vec), 256, 0, stream>>>(static_cast<const uint4*>(x_bf16), n_vec, reinterpret_cast<uint32_t*>(descale) + 1);
+    const bool wide = n_vec >= kWideVecs;
+    const unsigned grid = grid_for(n_vec, wide ? 4u : 1u);
+    if (wide) amax_kernel<4><<<grid, 256, 0, stream>>>(x, n_vec, reinterpret_cast<uint32_t*>(descale) + 1);
+    else amax_kernel<1><<<grid, 256, 0, stream>>>(x, n_vec, reinterpret_cast<uint32_t*>(descale) + 1);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    quantize_v_kernel<<<grid_for(n_vec), 256, 0, stream>>>(static_cast<const uint4*>(x_bf16), n_vec, static_cast<uint2*>(out_e4m3), descale);
-    return cudaGetLastError();
+    return launch_pdl(wide ? quantize_v_kernel<4> : quantize_v_kernel<1>, grid, 256u, stream, x, n_vec, out, descale);
 }
 
 }  // namespace b200mx

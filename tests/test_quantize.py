@@ -103,3 +103,39 @@ def test_quantise_then_attend_passes_the_gate(oracle):
     s = torch.einsum("bshd,bthd->bhst", qf, kf) / 128 ** 0.5
     want = torch.einsum("bhst,bthd->bshd", torch.softmax(s, -1), vf)
     assert (out.float() - want).abs().max().item() < 0.05
+
+
+def test_the_division_by_a_residual_rounds_like_a_division():
+    """The device quantiser of V divides by amax / 448 with a reciprocal and one residual correction. x and amax are bf16, so their 128 x 128
+    mantissas are all there is: the corrected quotient is the correctly rounded one for each."""
+    f32, f64 = np.float32, np.float64
+    x = (128 + np.arange(128)).astype(f32)[None, :]
+    vd = ((128 + np.arange(128)).astype(f32) / f32(448))[:, None]
+    r = f32(1) / vd
+    q = x * r
+    rem = (x.astype(f64) - q.astype(f64) * vd.astype(f64)).astype(f32)   # the products of two f32 and the difference are exact in f64
+    fixed = (q.astype(f64) + rem.astype(f64) * r.astype(f64)).astype(f32)
+    assert (q != x / vd).any() and np.array_equal(fixed, x / vd)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_vec", [1, 31, 8191, 8193, 32768, 32769, 1212416, 1212417])   # a cluster's registers full and one more; one and four loads per thread
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -110])   # the divisor inside the range of the correction, and below it
+def test_quantize_v_sizes(oracle, n_vec, scale):
+    torch = pytest.importorskip("torch")
+    from amdgpu_rustdsl_b200 import quantize_qk, quantize_v
+    x = (torch.randn(n_vec * 8, generator=torch.Generator().manual_seed(n_vec)) * scale).to(torch.bfloat16)
+    out, vs = torch.zeros(n_vec * 8, dtype=torch.uint8, device="cuda"), torch.zeros(1024, dtype=torch.float32, device="cuda")
+    quantize_v(x.cuda(), out, vs)
+    vd = (x.float().abs().max() / 448.0).item()
+    assert vs[0].item() == vd
+    want = (x.float() / vd).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
+    assert torch.equal(out.cpu(), want)
+    if n_vec % 16 == 0 and scale == 1.0:   # whole rows of 128: the Q / K quantiser at the same sizes
+        rows = n_vec // 16
+        y, s = torch.zeros(rows, 128, dtype=torch.uint8, device="cuda"), torch.zeros(rows * 4, dtype=torch.uint8, device="cuda")
+        quantize_qk(x.view(rows, 128).cuda(), y, s, mul=1.0)
+        f = x.view(rows, 4, 32).float()
+        e = (torch.frexp(f.abs().amax(-1)).exponent - 1 - 8 + 127).clamp(0, 254)
+        assert torch.equal(s.cpu().view(rows, 4).int(), e.int())
+        assert torch.equal(y.cpu(), torch.ldexp(f, (127 - e)[..., None]).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8).view(rows, 128))
