@@ -68,6 +68,9 @@ constexpr int kCols = 128;                  // score columns per softmax thread
 constexpr int kThreads = 32 * (4 + 8 + 4);   // 4 service warps, 8 softmax warps, 4 epilogue warps
 // The register file (64 K registers) is dealt out unevenly once the roles part: every thread starts with kMaxRegs, the service and the
 // epilogue warpgroups give most of theirs back and the two softmax warpgroups take them.
+#ifndef MXA_MIN_PART
+#define MXA_MIN_PART 2
+#endif
 #ifndef MXA_SERVICE_REGS
 #define MXA_SERVICE_REGS 56
 #define MXA_SOFTMAX_REGS 176
@@ -242,19 +245,27 @@ __device__ __forceinline__ void scale_tmem64(uint32_t taddr, float f) {
     tmem_st32(taddr + 32, b);
 }
 
-// One unit of work of the persistent kernel: 128 query rows of one (batch, head) against the key range of one split.
+// One unit of work of the persistent kernel: 128 query rows against the key range of one split. The rows are 128 of one (batch, head), or, with
+// the heads of a KV head packed (AttnParams::pack_shift), 128 >> pack_shift sequence rows of each of the 1 << pack_shift heads that share it:
+// TMEM lane r is then sequence row row0 + (r >> pack_shift) of head head + r % (1 << pack_shift).
 struct Item {
     uint32_t row0, head, batch, split, kv_head, key_lo, key_hi;
-    uint32_t half;   // 0: the item's whole key range; 1 / 2: its first / second half, to be merged with the other CTA of the cluster
+    uint32_t half;   // pairs: 0: the item's whole key range; 1 / 2: its first / second half, to be merged with the other CTA of the cluster
     int n_tiles;
 };
 
-template <bool kSplit, bool kCausal, bool kPair>
+// How a launch deals the key range of an item out within a cluster: not at all, the last round's items between pairs, every item between all CTAs.
+enum Cluster { kNoCluster = 0, kPairs = 1, kCutAll = 2 };
+
+template <bool kSplit, bool kCausal, Cluster kCluster, bool kPack>
 __device__ __forceinline__ Item decode_item(uint32_t w, const AttnParams& p) {
+    const uint32_t ps = kPack ? p.pack_shift : 0u;
     // w = (z * H + head) * n_qtiles + q tile: neighbouring CTAs work on neighbouring row blocks of one head, whose K / V they share in L2
     Item it;
     it.half = 0;
-    if (kPair && w >= p.tail_base) {   // a unit of the cut last round: half (w - tail_base) % 2 of item tail_base + (w - tail_base) / 2
+    const uint32_t part = w & ((1u << p.cut_log2) - 1u);   // kCutAll: unit w is part `part` of item w >> cut_log2
+    if (kCluster == kCutAll) w >>= p.cut_log2;
+    if (kCluster == kPairs && w >= p.tail_base) {   // a unit of the cut last round: half (w - tail_base) % 2 of item tail_base + (w - tail_base) / 2
         it.half = 1u + ((w - p.tail_base) & 1u);
         w = p.tail_base + ((w - p.tail_base) >> 1);
     }
@@ -272,9 +283,10 @@ __device__ __forceinline__ Item decode_item(uint32_t w, const AttnParams& p) {
         x = p.n_qtiles - 1u - rank / hb;
         yz = rank % hb;
     }
-    it.row0 = x * kRows;
-    it.head = yz % p.H;
-    const uint32_t z = yz / p.H;
+    it.row0 = x * (kRows >> ps);
+    const uint32_t hg = p.H >> ps;
+    it.head = (yz % hg) << ps;
+    const uint32_t z = yz / hg;
     it.batch = z;
     it.split = 0;
     if (kSplit) {
@@ -293,8 +305,14 @@ __device__ __forceinline__ Item decode_item(uint32_t w, const AttnParams& p) {
         it.key_hi = min(tile_hi * kKeys, p.SK);
     }
     // causal (crates/amdgpu-stage/src/attention/attn3.rs:298-306): row i sees the keys below min(i + SK - S + 1, SK); the item's last row decides
-    if (causal) it.key_hi = min(p.SK, it.row0 + kRows + (p.SK - p.S));
+    if (causal) it.key_hi = min(p.SK, it.row0 + (kRows >> ps) + (p.SK - p.S));
     it.n_tiles = (it.key_hi > it.key_lo) ? static_cast<int>((it.key_hi - it.key_lo + kKeys - 1) / kKeys) : 0;
+    if (kCluster == kCutAll) {   // every part has a tile: the launcher's rule
+        const uint32_t n = static_cast<uint32_t>(it.n_tiles), lo = (n * part) >> p.cut_log2, hi = (n * (part + 1u)) >> p.cut_log2;
+        it.key_hi = min(it.key_hi, it.key_lo + hi * kKeys);
+        it.key_lo += lo * kKeys;
+        it.n_tiles = static_cast<int>(hi - lo);
+    }
     if (it.half != 0u) {   // whole tiles [0, ceil(n / 2)) to the first half, the rest (and a ragged end) to the second
         const int first = (it.n_tiles + 1) / 2;
         if (it.half == 1u) {
@@ -315,13 +333,17 @@ __device__ __forceinline__ Item decode_item(uint32_t w, const AttnParams& p) {
 // two score tiles overlap the current item's last tiles and epilogue; only O is single: P V of an item's first tile waits until the
 // epilogue of the item before has read O out (o_free).
 // kTrace = false compiles every diagnostic (tile dumps, time stamps) out of the tile loop: the production launches use that variant.
-// kLazy: the long-sequence softmax recipe. kCausal: the causal mask (never with kSplit).
+// kLazy: the long-sequence softmax recipe. kCausal: the causal mask (never with kSplit). kCluster: only with kLazy.
+// kPack: AttnParams::pack_shift may be set. The row and head arithmetic of it cost 0.5 us an item where items are short, so the other launches have a
+// variant without.
 // kFused: the split kernel with the merge of the partials built into its epilogue (no pairs, no diagnostics, f16 partials, no peer routing).
-template <bool kSplit, bool kTrace, bool kLazy, bool kCausal, bool kPair, bool kVbs, bool kFused = false>
+template <bool kSplit, bool kTrace, bool kLazy, bool kCausal, Cluster kCluster, bool kVbs, bool kFused = false, bool kPack = kCluster != kNoCluster>
 __global__ void __maxnreg__(kMaxRegs)
 mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const AttnParams p) {
     auto stamp = [](float* trace, int role, int tile, int slot) { stamp_t<kTrace>(trace, role, tile, slot); };
+    constexpr bool kPair = kCluster == kPairs, kCut = kCluster == kCutAll;
+    const uint32_t pack_shift = kPack ? p.pack_shift : 0u;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -380,7 +402,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         }
         mbar_init(bar_o_free, kRows);   // the epilogue warpgroup's 128 threads
         mbar_init(bar_o_full, 1);
-        mbar_init(bar_peer_rdy, 1);
+        mbar_init(bar_peer_rdy, kCut ? 1u << p.cut_log2 : 1u);
         mbar_init(bar_peer_data, kRows);
         fence_mbar_init();
     }
@@ -408,10 +430,10 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    // launched as pairs (the last round's items are cut in two): the partner's barriers must exist before anything can arrive on them
+    // launched as clusters (items are cut between their CTAs): the partner's barriers must exist before anything can arrive on them
     // Every thread arrives on the cluster's barrier here and waits for it only where it first touches the partner (the epilogue
     // warpgroup, the score MMA warp) or, failing that, at the end; by then the partner has long arrived, so nobody stands still for it.
-    constexpr bool paired = kPair;
+    constexpr bool paired = kCluster != kNoCluster;
     bool cluster_joined = !paired;
     if (paired) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     auto join_cluster = [&]() {
@@ -454,7 +476,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             auto enter_item = [&](ScaleCursor& c) {
                 c.live = c.w < n_items;
                 if (!c.live) return;
-                const Item it = decode_item<kSplit, kCausal, kPair>(c.w, p);
+                const Item it = decode_item<kSplit, kCausal, kCluster, kPack>(c.w, p);
                 c.ptr = p.k_descale + static_cast<size_t>(it.batch) * p.ks_batch_stride + (static_cast<size_t>(it.key_lo + lane) * p.HK + it.kv_head) * 4u;
                 c.keys_left = static_cast<int>(p.SK - it.key_lo) - lane;
                 c.tiles_left = it.n_tiles;
@@ -482,15 +504,16 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             auto load_q_scales = [&](const Item& it, uint32_t (&w)[4]) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    uint32_t r = it.row0 + lane + 32 * i;
-                    r = min(r, p.S - 1u);   // rows past the sequence reuse the last row's scales (block3.rs:110-113)
-                    const size_t off = static_cast<size_t>(it.batch) * p.qs_batch_stride + (static_cast<size_t>(r) * p.H + it.head) * 4u;
+                    const uint32_t lr = lane + 32 * i;
+                    const uint32_t r = min(it.row0 + (lr >> pack_shift), p.S - 1u);   // rows past the sequence reuse the last row's scales (block3.rs:110-113)
+                    const uint32_t head = it.head + (lr & ((1u << pack_shift) - 1u));
+                    const size_t off = static_cast<size_t>(it.batch) * p.qs_batch_stride + (static_cast<size_t>(r) * p.H + head) * 4u;
                     w[i] = __ldg(reinterpret_cast<const uint32_t*>(p.q_descale + off));
                 }
             };
             // The CTA's first copies (Q tile and first K tile, first V tile of its first item) go out before anything else of the role's set-up.
             if (blockIdx.x < n_items && elect_one_sync()) {
-                const Item it = decode_item<kSplit, kCausal, kPair>(blockIdx.x, p);
+                const Item it = decode_item<kSplit, kCausal, kCluster, kPack>(blockIdx.x, p);
                 if (kIsK) {
                     mbar_arrive_expect_tx(bar_q_full(0), kTileBytes);
                     tma_load_4d(q_smem, &tm_q, bar_q_full(0), 0, static_cast<int>(it.head), static_cast<int>(it.row0), static_cast<int>(it.batch));
@@ -508,7 +531,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             enter_item(cs);
             if (kPar) advance(cs);   // this warp's first tile is the CTA's second
             uint32_t wq[4] = {0u, 0u, 0u, 0u}, w0[4], w1[4];
-            if (kIsK && blockIdx.x < n_items) load_q_scales(decode_item<kSplit, kCausal, kPair>(blockIdx.x, p), wq);
+            if (kIsK && blockIdx.x < n_items) load_q_scales(decode_item<kSplit, kCausal, kCluster, kPack>(blockIdx.x, p), wq);
             load_and_advance(cs, w0);
             load_and_advance(cs, w1);
 
@@ -516,7 +539,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             int st = 0;
             bool ok = true;
             for (uint32_t w = blockIdx.x; ok && w < n_items; w += stride, ++n) {
-                const Item it = decode_item<kSplit, kCausal, kPair>(w, p);
+                const Item it = decode_item<kSplit, kCausal, kCluster, kPack>(w, p);
                 const uint32_t qb = n & 1u;
                 if (kIsK) {
                     // the Q buffer was last used two items ago
@@ -532,7 +555,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     __syncwarp();
                     if (elect_one_sync()) mbar_arrive(bar_q_full(qb));
                     ++q_issued;
-                    if (w + stride < n_items) load_q_scales(decode_item<kSplit, kCausal, kPair>(w + stride, p), wq);   // the next item's Q scales, a whole item ahead
+                    if (w + stride < n_items) load_q_scales(decode_item<kSplit, kCausal, kCluster, kPack>(w + stride, p), wq);   // the next item's Q scales, a whole item ahead
                 }
                 float* k_trace = cta_traced ? p.trace : nullptr;   // stamps are indexed by the running tile counter
                 int key = static_cast<int>(it.key_lo);
@@ -630,12 +653,13 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             int st = 0;
             bool ok = true;
             for (uint32_t w = blockIdx.x; ok && w < n_items; w += stride, ++n) {
-                const Item qk_it = decode_item<kSplit, kCausal, kPair>(w, p);
+                const Item qk_it = decode_item<kSplit, kCausal, kCluster, kPack>(w, p);
                 const int n_tiles = qk_it.n_tiles;
                 const uint32_t qb = n & 1u;
                 float* mma_trace = cta_traced ? p.trace : nullptr;
                 // first half of a cut item: once its last score tile is done the K ring is idle for good, and the partner may push its
                 // half there (the commit below arrives on the partner's barrier)
+                if (kCut) join_cluster();   // (the same with the other CTAs of the cluster)
                 uint32_t partner_rdy = 0u;
                 if (kPair && qk_it.half == 1u) {
                     join_cluster();
@@ -670,6 +694,9 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         tc_commit(bar_k_empty(st));
                         if (j == n_tiles - 1) tc_commit(bar_q_empty(qb));   // the Q buffer can take the item after next
                         if (kPair && partner_rdy != 0u && j == n_tiles - 1) tc_commit(partner_rdy);
+                        if (kCut && j == n_tiles - 1) {
+                            for (uint32_t c = 0; c < (1u << p.cut_log2); ++c) tc_commit(map_to_cta(bar_peer_rdy, c));
+                        }
                         stamp(mma_trace, 2, static_cast<int>(g), 5);
                     }
                     ++g;
@@ -698,7 +725,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             int st = 0;
             bool ok = true;
             for (uint32_t w = blockIdx.x; ok && w < n_items; w += stride, ++n) {
-                const int n_tiles = decode_item<kSplit, kCausal, kPair>(w, p).n_tiles;
+                const int n_tiles = decode_item<kSplit, kCausal, kCluster, kPack>(w, p).n_tiles;
                 float* mma_trace = cta_traced ? p.trace : nullptr;
                 // an item's first tile overwrites O and L, which the epilogue of the item before must have read out
                 if (n > 0) ok = mbar_wait(bar_o_free, (n - 1u) & 1u, abort_flag);
@@ -781,7 +808,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             mbar_arrive(bar_p_full(par));
             p_ready = false;
         };
-        const bool want_fin = kSplit || p.lse_nat != nullptr || cta_traced || kPair;   // does anything read the final reference?
+        const bool want_fin = kSplit || p.lse_nat != nullptr || cta_traced || kCluster != kNoCluster;   // does anything read the final reference?
         float sf_held = 0.0f;   // log2 of the four block scales this group's buffer holds for the row, if they are equal
         auto scale_o = [&](float f) {
 #pragma unroll 1
@@ -797,13 +824,14 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             // the tile count, the number of tiles every row sees in full and the row's own key limit stay live through the tile loop
             int n_tiles, j_full, row_lim;   // row_lim: this row's visible keys, counted from the item's first key
             {
-                const Item it = decode_item<kSplit, kCausal, kPair>(w, p);
+                const Item it = decode_item<kSplit, kCausal, kCluster, kPack>(w, p);
                 n_tiles = it.n_tiles;
                 row_lim = static_cast<int>(it.key_hi - it.key_lo);
                 int first_lim = row_lim;   // the limit of the item's first row: the tiles below it need no mask
                 if (kCausal && !kSplit) {
-                    first_lim = min(row_lim, static_cast<int>(it.row0 + 1u + (p.SK - p.S)));
-                    row_lim = min(row_lim, static_cast<int>(it.row0 + r + 1u + (p.SK - p.S)));
+                    const int visible = static_cast<int>(it.row0 + 1u + (p.SK - p.S)) - static_cast<int>(it.key_lo);   // to the item's first row; none (<= 0) in a part behind its diagonal
+                    first_lim = max(min(row_lim, visible), 0);
+                    row_lim = min(row_lim, visible + static_cast<int>(r >> pack_shift));
                 }
                 j_full = first_lim / kKeys;
             }
@@ -1047,7 +1075,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const uint32_t t_o = tmem + kColO + lane_base, t_l = tmem + kColL + lane_base;
         const uint32_t stg = smem_base + SmemLayout::ostage;
         const bool issuer = threadIdx.x == 32u * kFirstEpilogueWarp;
-        const bool want_fin = kSplit || p.lse_nat != nullptr || cta_traced || kPair;
+        const bool want_fin = kSplit || p.lse_nat != nullptr || cta_traced || kCluster != kNoCluster;
         // Half items (the cut last round; a half item is a CTA's last unit, so its K / V rings are idle once its last P V is done): the CTA
         // with the first half tells its partner when its K ring is free (the commit of its last score tile arrives on the partner's
         // barrier); the partner pushes its unnormalised O (f32), row sums and references there with distributed-shared-memory stores and
@@ -1063,7 +1091,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         uint32_t n = 0;
         bool ok = true;
         for (uint32_t w = blockIdx.x; w < n_items; w += stride, ++n) {
-            const Item it = decode_item<kSplit, kCausal, kPair>(w, p);
+            const Item it = decode_item<kSplit, kCausal, kCluster, kPack>(w, p);
             const bool tracing = cta_traced && n == 0;
             const bool dumping = tracing && !(p.flags & 0x4u);
             float* ep_trace = (cta_traced && r == 0 && n < 6) ? p.trace : nullptr;   // epilogue stamps: P V role's row, tile index 24 + item ordinal, slots 0, 1, 5, 7
@@ -1106,6 +1134,91 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 mbar_arrive_remote(map_to_cta(bar_peer_data, 0u));
                 continue;
             }
+            if (kCut) {
+                // Every CTA of the cluster has a part of the item's keys. Row r is finished by CTA r % parts: all parts push the row's O (f32, not
+                // normalised), row sum and base there, into the K ring, which is idle in all of them once bar_peer_rdy has completed (the
+                // commits behind their last score tiles). A row goes out by its own thread, so its one arrival on the owner's barrier covers it;
+                // 128 rows' worth of arrivals is what every owner gets (128 / parts rows from each of the parts).
+                // Spreading the rows keeps the exchange at 64 KB in and out of every CTA whatever the number of parts, and rows past the
+                // sequence are not sent: a decode step exchanges a few rows.
+                const uint32_t lg = p.cut_log2, parts = 1u << lg, me = blockIdx.x & (parts - 1u);
+                join_cluster();
+                ok = mbar_wait_cluster(bar_peer_rdy, 0u, abort_flag);
+                if (!named_bar_all(kEpiBar, 128u, ok)) break;
+                auto cut_slot = [&](uint32_t source, uint32_t ro) { return (source << (7u - lg)) + ro; };   // row ro of the owner's, from part `source`
+                auto cut_off = [&](uint32_t quad, uint32_t ro) { return (quad >> 3) * 128u + (((quad & 7u) ^ (ro & 7u)) << 4); };   // 4 columns
+                {
+                    const uint32_t owner = r & (parts - 1u), ro = r >> lg, slot = cut_slot(me, ro);
+                    const uint32_t dst = map_to_cta(smem_base + SmemLayout::k + slot * 512u, owner);
+                    const bool live = it.row0 + (r >> pack_shift) < p.S;
+#pragma unroll
+                    for (uint32_t c = 0; c < 4; ++c) {
+                        uint32_t o[32];
+                        tmem_ld32(t_o + 32 * c, o);
+                        tmem_wait_ld();
+                        if (live) {
+#pragma unroll
+                            for (uint32_t q4 = 0; q4 < 8; ++q4) {
+                                asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst + cut_off(8u * c + q4, ro)),
+                                             "r"(o[4 * q4]), "r"(o[4 * q4 + 1]), "r"(o[4 * q4 + 2]), "r"(o[4 * q4 + 3]) : "memory");
+                            }
+                        }
+                    }
+                    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(map_to_cta(smem_base + SmemLayout::xstat + slot * 8u, owner)), "f"(l), "f"(ref_fin) : "memory");
+                    mbar_arrive_remote(map_to_cta(bar_peer_data, owner));
+                }
+                ok = mbar_wait_cluster(bar_peer_data, 0u, abort_flag);
+                if (!named_bar_all(kEpiBar, 128u, ok)) break;
+                // `parts` threads share an owned row, a thread takes every parts-th group of 4 columns
+                const uint32_t et = threadIdx.x - 32u * kFirstEpilogueWarp, ro = et >> lg, c0 = et & (parts - 1u);
+                const uint32_t mr = (ro << lg) + me, row = it.row0 + (mr >> pack_shift), head = it.head + (mr & ((1u << pack_shift) - 1u));
+                if (row < p.S) {
+                    auto stat = [&](uint32_t source) {
+                        float2 ps;   // {row sum, base}
+                        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(ps.x), "=f"(ps.y) : "r"(smem_base + SmemLayout::xstat + cut_slot(source, ro) * 8u) : "memory");
+                        return ps;
+                    };
+                    // the bases are integers: the weights are exact powers of two (0 for a part without a visible key, whose base is -inf)
+                    float base = -INFINITY, sum = 0.0f;
+                    for (uint32_t c = 0; c < parts; ++c) base = fmaxf(base, stat(c).y);
+                    for (uint32_t c = 0; c < parts; ++c) {
+                        const float2 ps = stat(c);
+                        sum += ps.x * ex2_approx(ps.y - base);
+                    }
+                    const float fin = vd / sum;
+                    const size_t prow = (static_cast<size_t>(it.batch) * p.S + row) * p.H + head + (kSplit ? static_cast<size_t>(it.split) * p.rows_total : 0u);
+                    uint8_t* dst = kSplit ? static_cast<uint8_t*>(p.ohat) + prow * 256u
+                                          : p.o + static_cast<size_t>(it.batch) * p.o_batch_stride + static_cast<size_t>(row) * p.o_row_stride + static_cast<size_t>(head) * p.o_head_stride;
+                    for (uint32_t quad = c0; quad < 32u; quad += parts) {
+                        float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        for (uint32_t c = 0; c < parts; ++c) {
+                            const float f = ex2_approx(stat(c).y - base);
+                            float4 pb;
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(pb.x), "=f"(pb.y), "=f"(pb.z), "=f"(pb.w)
+                                         : "r"(smem_base + SmemLayout::k + cut_slot(c, ro) * 512u + cut_off(quad, ro)) : "memory");
+                            acc.x = fmaf(pb.x, f, acc.x);
+                            acc.y = fmaf(pb.y, f, acc.y);
+                            acc.z = fmaf(pb.z, f, acc.z);
+                            acc.w = fmaf(pb.w, f, acc.w);
+                        }
+                        uint2 wv;
+                        if (kSplit) {
+                            asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(wv.x) : "f"(acc.y * fin), "f"(acc.x * fin));
+                            asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(wv.y) : "f"(acc.w * fin), "f"(acc.z * fin));
+                        } else {
+                            const __nv_bfloat162 b01 = __floats2bfloat162_rn(acc.x * fin, acc.y * fin), b23 = __floats2bfloat162_rn(acc.z * fin, acc.w * fin);
+                            wv = make_uint2(*reinterpret_cast<const uint32_t*>(&b01), *reinterpret_cast<const uint32_t*>(&b23));
+                        }
+                        *reinterpret_cast<uint2*>(dst + quad * 8u) = wv;
+                    }
+                    if (c0 == 0u) {
+                        const float lse2 = base - kPOffset + lg2_approx(sum);
+                        if (kSplit) p.lse2[prow] = lse2;
+                        else if (p.lse_nat != nullptr) p.lse_nat[(static_cast<size_t>(it.batch) * p.H + head) * p.S + row] = lse2 * 0.6931471805599453f;
+                    }
+                }
+                continue;   // (a CTA's only unit)
+            }
             float fa = 1.0f, fb = 0.0f;   // weights of the own and of the partner's half in a merge
             if (kPair && it.half == 1u) {
                 join_cluster();
@@ -1119,7 +1232,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 l = l * fa + ps.x * fb;
             }
             const float fin = vd / l;
-            const uint32_t row = it.row0 + r;
+            const uint32_t row = it.row0 + (r >> pack_shift), head = it.head + (r & ((1u << pack_shift) - 1u));
             if (tracing) {
                 p.trace[32768 + r] = l;
                 p.trace[32768 + 128 + r] = ref_out;
@@ -1261,12 +1374,12 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 const float lse2 = ref_out - kPOffset + lg2_approx(l);   // log2 of sum_j 2^(s_j)
                 if (kSplit && !kFused && p.peer != nullptr) {
                     const uint32_t dest = it.row0 / p.peer->dest_rows, n_rows = p.peer->dest_rows * p.H;
-                    p.peer->lse[dest][static_cast<size_t>(p.peer->rank) * n_rows + static_cast<size_t>(row - dest * p.peer->dest_rows) * p.H + it.head] = lse2;
+                    p.peer->lse[dest][static_cast<size_t>(p.peer->rank) * n_rows + static_cast<size_t>(row - dest * p.peer->dest_rows) * p.H + head] = lse2;
                 } else if (kSplit) {
-                    const size_t prow = static_cast<size_t>(it.split) * p.rows_total + (static_cast<size_t>(it.batch) * p.S + row) * p.H + it.head;
+                    const size_t prow = static_cast<size_t>(it.split) * p.rows_total + (static_cast<size_t>(it.batch) * p.S + row) * p.H + head;
                     p.lse2[prow] = lse2;
                 } else if (p.lse_nat != nullptr) {
-                    p.lse_nat[(static_cast<size_t>(it.batch) * p.H + it.head) * p.S + row] = lse2 * 0.6931471805599453f;
+                    p.lse_nat[(static_cast<size_t>(it.batch) * p.H + head) * p.S + row] = lse2 * 0.6931471805599453f;
                 }
             }
             if (kFused) {
@@ -1393,9 +1506,11 @@ cudaError_t launch_attention(const CUtensorMap& tm_q, const CUtensorMap& tm_k, c
     using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const AttnParams);
     // The instantiations: [causal][recipe][trace][split] (the causal mask has no split form); behind them the variants for launches as pairs
     // of CTAs (long-sequence recipe, no mask): [trace][split]; behind those the variants with V block scales (no mask, no trace):
-    // [pair][recipe][split], pairs only with the long-sequence recipe; last the split kernels with the fused merge: [V block scales][recipe].
-#define MXA_K(split, trace, lazy, causal, pair, vbs) mxfp8_prefill_kernel<split, trace, lazy, causal, pair, vbs>
-    static const Kernel kernels[32] = {
+    // [pair][recipe][split], pairs only with the long-sequence recipe; then the split kernels with the fused merge: [V block scales][recipe];
+    // then the variants that cut every item between the CTAs of a cluster: [V block scales][split], and the causal one;
+    // last the variants with packed heads (the clusters' all have them): unsplit [none, causal, V block scales][recipe], split [V block scales][recipe].
+#define MXA_K(split, trace, lazy, causal, pair, vbs) mxfp8_prefill_kernel<split, trace, lazy, causal, pair ? kPairs : kNoCluster, vbs>
+    static const Kernel kernels[47] = {
         MXA_K(false, false, false, false, false, false), MXA_K(true, false, false, false, false, false), MXA_K(false, true, false, false, false, false),
         MXA_K(true, true, false, false, false, false),   MXA_K(false, false, true, false, false, false), MXA_K(true, false, true, false, false, false),
         MXA_K(false, true, true, false, false, false),   MXA_K(true, true, true, false, false, false),   MXA_K(false, false, false, true, false, false),
@@ -1407,17 +1522,27 @@ cudaError_t launch_attention(const CUtensorMap& tm_q, const CUtensorMap& tm_k, c
         MXA_K(false, false, false, false, false, true),  MXA_K(true, false, false, false, false, true),  MXA_K(false, false, true, false, false, true),
         MXA_K(true, false, true, false, false, true),    nullptr,                                        nullptr,
         MXA_K(false, false, true, false, true, true),    MXA_K(true, false, true, false, true, true),
-        mxfp8_prefill_kernel<true, false, false, false, false, false, true>, mxfp8_prefill_kernel<true, false, true, false, false, false, true>,
-        mxfp8_prefill_kernel<true, false, false, false, false, true, true>,  mxfp8_prefill_kernel<true, false, true, false, false, true, true>};
+        mxfp8_prefill_kernel<true, false, false, false, kNoCluster, false, true>, mxfp8_prefill_kernel<true, false, true, false, kNoCluster, false, true>,
+        mxfp8_prefill_kernel<true, false, false, false, kNoCluster, true, true>,  mxfp8_prefill_kernel<true, false, true, false, kNoCluster, true, true>,
+        mxfp8_prefill_kernel<false, false, true, false, kCutAll, false>,     mxfp8_prefill_kernel<true, false, true, false, kCutAll, false>,
+        mxfp8_prefill_kernel<false, false, true, false, kCutAll, true>,      mxfp8_prefill_kernel<true, false, true, false, kCutAll, true>,
+        mxfp8_prefill_kernel<false, false, true, true, kCutAll, false>,
+#define MXA_PACKED(split, lazy, causal, vbs) mxfp8_prefill_kernel<split, false, lazy, causal, kNoCluster, vbs, false, true>
+        MXA_PACKED(false, false, false, false), MXA_PACKED(false, true, false, false), MXA_PACKED(false, false, true, false), MXA_PACKED(false, true, true, false),
+        MXA_PACKED(false, false, false, true),  MXA_PACKED(false, true, false, true),  MXA_PACKED(true, false, false, false), MXA_PACKED(true, true, false, false),
+        MXA_PACKED(true, false, false, true),   MXA_PACKED(true, true, false, true)};
+#undef MXA_PACKED
 #undef MXA_K
-    constexpr int kKernels = 32;
+    constexpr int kKernels = 47, kFirstCut = 32, kFirstPacked = 37, kCutLogs = 5;   // cut between up to 16 CTAs
     constexpr int kMaxDevices = 64;
     // per-device set-up done lazily from whichever thread launches first: plain flags would be a data race, and both steps are idempotent
     static std::atomic<bool> attr_done[kMaxDevices][kKernels];   // the shared-memory attribute is per device
     static std::atomic<int> sm_count[kMaxDevices];
     static std::atomic<int> pair_capacity[kMaxDevices][kKernels];   // -1 = not asked yet (set below on first use)
+    static std::atomic<int> cut_capacity[kMaxDevices][kFirstPacked - kFirstCut][kCutLogs];   // [.][.][log2 of the cluster's CTAs]
     static std::once_flag pair_init;
     std::call_once(pair_init, [] {
+        for (auto& d : cut_capacity) for (auto& k : d) for (auto& x : k) x.store(-1, std::memory_order_relaxed);
         for (auto& d : pair_capacity) for (auto& x : d) x.store(-1, std::memory_order_relaxed);
     });
     // the long-sequence recipe from 4 key tiles of the whole sequence on (crates/amdgpu-stage/src/attention/state.rs:73-77), unless the
@@ -1431,6 +1556,10 @@ cudaError_t launch_attention(const CUtensorMap& tm_q, const CUtensorMap& tm_k, c
     const bool fused = p.fused_counters != nullptr;
     if (fused && (!split || p.trace != nullptr || p.peer != nullptr || (p.flags & kFlagF32Partials) || p.splits > 8u || p.o == nullptr)) return cudaErrorInvalidValue;
     if (fused) which = 28 + (lazy_recipe ? 1 : 0) + (vbs ? 2 : 0);
+    if (p.pack_shift != 0u) {
+        if (p.trace != nullptr || p.peer != nullptr || fused) return cudaErrorInvalidValue;
+        which = kFirstPacked + (lazy_recipe ? 1 : 0) + (split ? 6 + (vbs ? 2 : 0) : (causal ? 2 : 0) + (vbs ? 4 : 0));
+    }
     const int which_pair = vbs ? 26 + (split ? 1 : 0) : 16 + (split ? 1 : 0) + (p.trace != nullptr ? 2 : 0);   // only for the long-sequence recipe without a mask
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -1438,7 +1567,9 @@ cudaError_t launch_attention(const CUtensorMap& tm_q, const CUtensorMap& tm_k, c
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     auto ensure_attr = [&](int k) -> cudaError_t {
         if (attr_done[dev][k].load(std::memory_order_acquire)) return cudaSuccess;
-        const cudaError_t ea = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernels[k]), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        cudaError_t ea = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernels[k]), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        if (ea == cudaSuccess && k >= kFirstCut && k < kFirstPacked)
+            ea = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernels[k]), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);   // 16 CTAs, where they fit
         if (ea == cudaSuccess) attr_done[dev][k].store(true, std::memory_order_release);
         return ea;
     };
@@ -1455,8 +1586,9 @@ cudaError_t launch_attention(const CUtensorMap& tm_q, const CUtensorMap& tm_k, c
     // Persistent launch: one CTA per SM (a CTA takes all of an SM's tensor memory and nearly all of its shared memory), each walking the
     // work units blockIdx.x, blockIdx.x + gridDim.x, ...
     AttnParams q = p;
-    q.n_qtiles = (p.S + kRows - 1) / kRows;
-    const unsigned long long items = 1ull * q.n_qtiles * p.H * B * (split ? p.splits : 1u);
+    const uint32_t seq_rows = kRows >> p.pack_shift;   // sequence rows of an item
+    q.n_qtiles = (p.S + seq_rows - 1) / seq_rows;
+    const unsigned long long items = 1ull * q.n_qtiles * (p.H >> p.pack_shift) * B * (split ? p.splits : 1u);
     if (items == 0 || items > 0x7FFFFFFFull) return cudaErrorInvalidValue;
     q.n_items = static_cast<uint32_t>(items);
     q.n_work = q.n_items;
@@ -1476,34 +1608,62 @@ cudaError_t launch_attention(const CUtensorMap& tm_q, const CUtensorMap& tm_k, c
     }
     const uint32_t even_sms = static_cast<uint32_t>(sms) & ~1u;
     constexpr uint32_t kMinTilesForPairs = 48u;
-    if (lazy_recipe && !causal && !fused && min_tiles >= kMinTilesForPairs && even_sms >= 2u && !(p.flags & kFlagNoTailSplit)) {
+    constexpr uint32_t kMinTilesPerPart = MXA_MIN_PART;
+    // how many clusters of `cluster` CTAs of kernel k the device holds at once (asked once per device, kernel and size, and kept in `known`)
+    auto clusters_that_fit = [&](int k, uint32_t cluster, std::atomic<int>& known) -> uint32_t {
+        int n = known.load(std::memory_order_relaxed);
+        if (n < 0) {
+            cudaLaunchConfig_t probe = {};
+            probe.gridDim = dim3(static_cast<uint32_t>(sms) / cluster * cluster, 1, 1);
+            probe.blockDim = dim3(kThreads, 1, 1);
+            probe.dynamicSmemBytes = kSmemBytes;
+            cudaLaunchAttribute pa[1];
+            pa[0].id = cudaLaunchAttributeClusterDimension;
+            pa[0].val.clusterDim.x = cluster; pa[0].val.clusterDim.y = 1; pa[0].val.clusterDim.z = 1;
+            probe.attrs = pa;
+            probe.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&n, reinterpret_cast<const void*>(kernels[k]), &probe) != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
+            known.store(n, std::memory_order_relaxed);
+        }
+        return static_cast<uint32_t>(n);
+    };
+    uint32_t cluster_ctas = 1u;
+    // Few items: each is cut between the CTAs of a cluster as long as the machine holds the clusters at once and every part keeps kMinTilesPerPart
+    // key tiles. The merge stays in shared memory, with f32 partials and no workspace.
+    const bool plain = p.trace == nullptr && p.peer == nullptr && !fused && !(p.flags & (kFlagF32Partials | kFlagNoTailSplit));
+    if (lazy_recipe && plain && 2u * q.n_items <= static_cast<uint32_t>(sms)) {
+        uint32_t tiles = min_tiles;
+        if (causal) tiles = (min(p.SK, seq_rows + (p.SK - p.S)) + kKeys - 1) / kKeys;   // the first row block's
+        const int k_cut = causal ? kFirstCut + 4 : kFirstCut + (split ? 1 : 0) + (vbs ? 2 : 0);
+        uint32_t lg = 0;
+        while (lg + 1 < kCutLogs && (q.n_items << (lg + 1)) <= static_cast<uint32_t>(sms) && tiles >= (kMinTilesPerPart << (lg + 1))) ++lg;
+        if (lg > 0) {
+            e = ensure_attr(k_cut);
+            if (e != cudaSuccess) return e;
+        }
+        while (lg > 0 && clusters_that_fit(k_cut, 1u << lg, cut_capacity[dev][k_cut - kFirstCut][lg]) < q.n_items) --lg;
+        if (lg > 0) {
+            q.cut_log2 = lg;
+            cluster_ctas = 1u << lg;
+            q.n_work = q.n_items << lg;
+            q.tail_base = q.n_work;
+            ctas = q.n_work;
+            which = k_cut;
+        }
+    }
+    if (cluster_ctas == 1u && lazy_recipe && !causal && !fused && min_tiles >= kMinTilesForPairs && even_sms >= 2u && !(p.flags & kFlagNoTailSplit)) {
         const uint32_t rounds = q.n_items / even_sms, tail = q.n_items - rounds * even_sms;
         if (tail > 0u && 2u * tail <= even_sms) {
             const uint32_t grid = rounds > 0u ? even_sms : 2u * tail;
             e = ensure_attr(which_pair);
             if (e != cudaSuccess) return e;
-            int max_clusters = pair_capacity[dev][which_pair].load(std::memory_order_relaxed);
-            if (max_clusters < 0) {   // how many pairs of CTAs of this kernel the device holds at once (asked once per device and kernel)
-                cudaLaunchConfig_t probe = {};
-                probe.gridDim = dim3(even_sms, 1, 1);
-                probe.blockDim = dim3(kThreads, 1, 1);
-                probe.dynamicSmemBytes = kSmemBytes;
-                cudaLaunchAttribute pa[1];
-                pa[0].id = cudaLaunchAttributeClusterDimension;
-                pa[0].val.clusterDim.x = 2; pa[0].val.clusterDim.y = 1; pa[0].val.clusterDim.z = 1;
-                probe.attrs = pa;
-                probe.numAttrs = 1;
-                int n = 0;
-                if (cudaOccupancyMaxActiveClusters(&n, reinterpret_cast<const void*>(kernels[which_pair]), &probe) != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
-                max_clusters = n;
-                pair_capacity[dev][which_pair].store(n, std::memory_order_relaxed);
-            }
-            if (static_cast<uint32_t>(max_clusters) * 2u >= grid) {
+            if (clusters_that_fit(which_pair, 2u, pair_capacity[dev][which_pair]) * 2u >= grid) {
                 q.tail_split = 1u;
                 q.tail_base = rounds * even_sms;
                 q.n_work = q.tail_base + 2u * tail;
                 ctas = grid;
                 which = which_pair;
+                cluster_ctas = 2u;
             }
         }
     }
@@ -1517,9 +1677,9 @@ cudaError_t launch_attention(const CUtensorMap& tm_q, const CUtensorMap& tm_k, c
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (q.tail_split != 0u) {
+    if (cluster_ctas > 1u) {
         attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+        attr[1].val.clusterDim.x = cluster_ctas; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
         cfg.numAttrs = 2;
     }
     return cudaLaunchKernelEx(&cfg, kernels[which], tm_q, tm_k, tm_v, tm_o, q);

@@ -151,15 +151,15 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// A [batch, seq, heads, 128] e4m3 tensor as a 4-D map (head dim, head, row, batch) with a box of `box_rows` rows x 128 bytes, 128-byte
-// swizzle. Rows past `seq` read as zero.
+// A [batch, seq, heads, 128] e4m3 tensor as a 4-D map (head dim, head, row, batch) with a box of `box_rows` rows of `box_heads` heads x 128 bytes
+// (in shared memory the head is the faster index), 128-byte swizzle. Rows past `seq` read as zero.
 int make_tile_map(CUtensorMap* m, const void* base, uint64_t seq, uint64_t heads, uint64_t batches, uint64_t head_stride, uint64_t row_stride,
-                  uint64_t batch_stride, uint32_t box_rows) {
+                  uint64_t batch_stride, uint32_t box_rows, uint32_t box_heads = 1) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return -static_cast<int>(cudaErrorSymbolNotFound);
     const cuuint64_t dims[4] = {128, heads, seq, batches};
     const cuuint64_t strides[3] = {head_stride, row_stride, batch_stride == 0 ? row_stride * seq : batch_stride};
-    const cuuint32_t box[4] = {128, 1, box_rows, 1};
+    const cuuint32_t box[4] = {128, box_heads, box_rows, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -167,14 +167,14 @@ int make_tile_map(CUtensorMap* m, const void* base, uint64_t seq, uint64_t heads
 }
 
 // The bf16 output [batch, seq, heads, 128] as a 4-D map (head dim, head, row, batch) with a 128-row x 64-column box, 128-byte swizzle:
-// the shape of one warpgroup's TMA store. Rows past `seq` are not written.
+// the shape of one warpgroup's TMA store (the 128 rows: 128 / box_heads sequence rows of box_heads heads). Rows past `seq` are not written.
 int make_out_map(CUtensorMap* m, void* base, uint64_t seq, uint64_t heads, uint64_t batches, uint64_t head_stride, uint64_t row_stride,
-                 uint64_t batch_stride) {
+                 uint64_t batch_stride, uint32_t box_heads) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return -static_cast<int>(cudaErrorSymbolNotFound);
     const cuuint64_t dims[4] = {128, heads, seq, batches};
     const cuuint64_t strides[3] = {head_stride, row_stride, batch_stride == 0 ? row_stride * seq : batch_stride};
-    const cuuint32_t box[4] = {64, 1, 128, 1};
+    const cuuint32_t box[4] = {64, box_heads, 128 / box_heads, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -182,14 +182,15 @@ int make_out_map(CUtensorMap* m, void* base, uint64_t seq, uint64_t heads, uint6
 }
 
 // The split kernel's partials [splits][B*S*H rows][128] as a 5-D map (head dim, head, row, batch, split), 128-byte swizzle: f16 rows of
-// 256 bytes with a 128-row x 64-column box, or f32 rows of 512 bytes with a 128-row x 32-column box (either box is 128 bytes wide).
-int make_partial_map(CUtensorMap* m, void* base, uint64_t seq, uint64_t heads, uint64_t batches, uint64_t splits, bool f32) {
+// 256 bytes with a 128-row x 64-column box, or f32 rows of 512 bytes with a 128-row x 32-column box (either box is 128 bytes wide; its rows are
+// 128 / box_heads sequence rows of box_heads heads).
+int make_partial_map(CUtensorMap* m, void* base, uint64_t seq, uint64_t heads, uint64_t batches, uint64_t splits, bool f32, uint32_t box_heads = 1) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return -static_cast<int>(cudaErrorSymbolNotFound);
     const uint64_t rb = f32 ? 512 : 256;
     const cuuint64_t dims[5] = {128, heads, seq, batches, splits};
     const cuuint64_t strides[4] = {rb, heads * rb, seq * heads * rb, batches * seq * heads * rb};
-    const cuuint32_t box[5] = {f32 ? 32u : 64u, 1, 128, 1, 1};
+    const cuuint32_t box[5] = {f32 ? 32u : 64u, box_heads, 128 / box_heads, 1, 1};
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     const CUresult r = enc(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -219,7 +220,8 @@ int launch_attention_kernel(int kernel, const void* args, const uint32_t grid[3]
     p.gqa_shift = log2_u32(a->s_gqa);
     p.o = static_cast<uint8_t*>(a->ptr_o);
     p.o_row_stride = a->s_o_Seqs;
-    p.o_batch_stride = a->s_o_Bs;
+    p.o_batch_stride = a->s_o_Bs == 0u ? a->s_o_Seqs * p.S : a->s_o_Bs;   // 0: the rows of the batch elements follow each other (make_out_map)
+    p.o_head_stride = a->s_o_Hs;
     p.q_descale = static_cast<const uint8_t*>(a->ptr_q_descale);
     p.k_descale = static_cast<const uint8_t*>(a->ptr_k_descale);
     p.v_descale = static_cast<const float*>(a->ptr_v_descale);
@@ -261,13 +263,22 @@ int launch_attention_kernel(int kernel, const void* args, const uint32_t grid[3]
         }
     }
     if (split && static_cast<uint64_t>(p.rows_total) != static_cast<uint64_t>(B) * p.S * p.H) return FMHA_MXFP8_E_KA_IS;
-    // The four tensor maps depend on nothing but the argument block (pointers, extents, strides, flags): a call with the bytes of an
+    // Grouped heads: the query rows of all the heads of a KV head can share the 128-row items, since they meet the same keys. An item is the same
+    // work either way, so the heads are packed when that gives fewer items: a decode step of one row and four heads per KV head has a quarter of
+    // them, a prompt whose length is a multiple of 128 as many, and those stay as they were.
+    p.pack_shift = 0;
+    if (p.gqa_shift >= 1u && p.gqa_shift <= 4u && p.trace == nullptr && p.peer == nullptr && p.fused_counters == nullptr) {
+        const uint64_t seq_rows = 128u >> p.gqa_shift;
+        if ((p.S + seq_rows - 1) / seq_rows < ((static_cast<uint64_t>(p.S) + 127) / 128 << p.gqa_shift)) p.pack_shift = p.gqa_shift;
+    }
+    const uint32_t box_heads = 1u << p.pack_shift;
+    // The four tensor maps depend on nothing but the argument block (pointers, extents, strides, flags) and the packing: a call with the bytes of an
     // earlier one reuses its maps instead of encoding them again (four driver calls; a framework calls a layer with the same buffers
     // step after step). A few entries, replaced in turn; the lock is held for two short copies.
     struct MapSet {
         bool valid;
         int kernel;
-        uint32_t grid_z;
+        uint32_t grid_z, pack_shift;
         unsigned char args[sizeof(fmha_mxfp8_attn_args) > sizeof(fmha_mxfp8_kvsplit_args) ? sizeof(fmha_mxfp8_attn_args) : sizeof(fmha_mxfp8_kvsplit_args)];
         CUtensorMap tq, tk, tv, to;
     };
@@ -282,21 +293,21 @@ int launch_attention_kernel(int kernel, const void* args, const uint32_t grid[3]
         std::lock_guard<std::mutex> g(sets_lock);
         for (int i = 0; i < kMapSets && !have; ++i) {
             const MapSet& m = sets[i];
-            if (m.valid && m.kernel == kernel && m.grid_z == grid[2] && std::memcmp(m.args, args, arg_bytes) == 0) {
+            if (m.valid && m.kernel == kernel && m.grid_z == grid[2] && m.pack_shift == p.pack_shift && std::memcmp(m.args, args, arg_bytes) == 0) {
                 tq = m.tq; tk = m.tk; tv = m.tv; to = m.to;
                 have = true;
             }
         }
     }
     if (!have) {
-        int r = make_tile_map(&tq, a->ptr_q, p.S, p.H, B, a->s_Hs, a->s_Seqs, a->s_Bs, 128u);
+        int r = make_tile_map(&tq, a->ptr_q, p.S, p.H, B, a->s_Hs, a->s_Seqs, a->s_Bs, 128u / box_heads, box_heads);
         if (r) return r;
         r = make_tile_map(&tk, a->ptr_k, p.SK, p.HK, B, a->s_k_Hs, a->s_k_Seqs, a->s_k_Bs, b200mx::kKeysPerTile);
         if (r) return r;
         r = make_tile_map(&tv, a->ptr_v, p.SK, p.HK, B, a->s_v_Hs, a->s_v_Seqs, a->s_v_Bs, b200mx::kKeysPerTile);
         if (r) return r;
-        if (!split) r = make_out_map(&to, a->ptr_o, p.S, p.H, B, a->s_o_Hs, a->s_o_Seqs, a->s_o_Bs);
-        else r = make_partial_map(&to, p.ohat, p.S, p.H, B, p.splits, (p.flags & FMHA_MXFP8_FLAG_F32_PARTIALS) != 0u);
+        if (!split) r = make_out_map(&to, a->ptr_o, p.S, p.H, B, a->s_o_Hs, a->s_o_Seqs, a->s_o_Bs, box_heads);
+        else r = make_partial_map(&to, p.ohat, p.S, p.H, B, p.splits, (p.flags & FMHA_MXFP8_FLAG_F32_PARTIALS) != 0u, box_heads);
         if (r) return r;
         std::lock_guard<std::mutex> g(sets_lock);
         MapSet& m = sets[next_set];
@@ -304,6 +315,7 @@ int launch_attention_kernel(int kernel, const void* args, const uint32_t grid[3]
         m.valid = true;
         m.kernel = kernel;
         m.grid_z = grid[2];
+        m.pack_shift = p.pack_shift;
         std::memcpy(m.args, args, arg_bytes);
         m.tq = tq; m.tk = tk; m.tv = tv; m.to = to;
     }

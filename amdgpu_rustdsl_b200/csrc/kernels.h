@@ -43,7 +43,10 @@ struct AttnParams {
     const PeerPlan* peer;         // extension (split kernel, B = 1): store the partial rows to the GPUs that combine them (the plan's maps must be of the launch's partial format); may be null
     // shape
     uint32_t S, SK, H, HK, gqa_shift;
-    uint32_t o_row_stride, o_batch_stride;    // bytes
+    // 0, or gqa_shift: an item's 128 rows are 128 >> pack_shift sequence rows of all the heads of one KV head (the Q and output maps' boxes must
+    // be of that shape). Not with the diagnostics, the fused merge or a routing plan.
+    uint32_t pack_shift;
+    uint32_t o_row_stride, o_batch_stride, o_head_stride;    // bytes
     uint32_t qs_batch_stride, ks_batch_stride;  // bytes
     uint32_t splits, split_log2, rows_total;
     uint32_t flags;
@@ -51,14 +54,16 @@ struct AttnParams {
     // [, split])); the CTAs walk work units 0 .. n_work-1. Units below tail_base are whole items. With tail_split the items of the last,
     // partly filled round are cut in two key ranges each: unit tail_base + 2 i + h is half h of item tail_base + i, and the two CTAs of a
     // cluster take the two halves of one item and merge them through distributed shared memory
-    uint32_t n_qtiles, n_items, n_work, tail_base, tail_split;
+    // With cut_log2 > 0 every item is cut in 1 << cut_log2 key ranges instead: unit (i << cut_log2) + c is part c of item i, the CTAs of a cluster take
+    // the parts of one item and a CTA has one unit.
+    uint32_t n_qtiles, n_items, n_work, tail_base, tail_split, cut_log2;
     // diagnostics
     float* trace;          // may be null
     uint32_t* status;      // device status word
 };
 
 // rows_per_cta is 128 (t128) or 256 (vs128 / kvsplit): the logical block height of the reference's grids.
-// tm_o: the target of the kernel's TMA stores: the bf16 output as a 4-D map with a 128-row x 64-column box (unsplit kernels), or the
+// tm_o: the target of the kernel's TMA stores: the bf16 output as a 4-D map with a 128-row x 64-column box (unsplit kernels; rows = sequence rows x packed heads), or the
 // partials as a 5-D map (split kernel): f16 with a 128-row x 64-column box, or f32 with a 128-row x 32-column box
 cudaError_t launch_attention(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_o, const AttnParams& p,
                              uint32_t B, bool split, uint32_t rows_per_cta, cudaStream_t stream);

@@ -1,0 +1,96 @@
+"""Query heads of a KV head packed into one row block, and row blocks cut between the CTAs of a cluster: against the same call with every head on
+its own K and V (nothing to pack) and with FMHA_MXFP8_FLAG_NO_TAIL_SPLIT (nothing cut), which the other GPU tests hold against the fp64 oracle."""
+import math
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(B, H, HK, S, SK, seed=3):
+    from amdgpu_rustdsl_b200 import Q_PRESCALE, quantize_qk, quantize_v
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    q, k, v = (torch.randn(shape, generator=g, device="cuda").to(torch.bfloat16) for shape in ((B, S, H, 128), (B, SK, HK, 128), (B, SK, HK, 128)))
+    q *= torch.linspace(0.5, 3.0, H, device="cuda")[:, None].to(torch.bfloat16)
+    q8, k8, v8 = (torch.empty(x.shape, dtype=torch.uint8, device="cuda") for x in (q, k, v))
+    qs = torch.zeros(B * S * H * 4 + 512 * H * 4, dtype=torch.uint8, device="cuda")
+    ks = torch.zeros(B * SK * HK * 4 + 640 * H * 4, dtype=torch.uint8, device="cuda")
+    vs = torch.zeros(1024, dtype=torch.float32, device="cuda")
+    quantize_qk(q, q8, qs, mul=Q_PRESCALE)
+    quantize_qk(k, k8, ks)
+    quantize_v(v, v8, vs)
+    vb = torch.randint(120, 128, (B, -(-SK // 32), HK, 128), generator=g, device="cuda", dtype=torch.uint8)
+    return q8, k8, v8, qs, ks, vs, vb
+
+
+def _run(d, path, splits, causal, vblocks, flags):
+    from amdgpu_rustdsl_b200 import device_status, fmha_fwd_mxfp8
+    q, k, v, qs, ks, vs, vb = d
+    B, S, H, _ = q.shape
+    out = torch.full((B, S, H, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    lse = torch.full((B, H, S), float("nan"), device="cuda") if path != "kvsplit" else None
+    fmha_fwd_mxfp8(q, k, v, qs, ks, vs, out, path=path, splits=splits, causal=causal, flags=flags, lse=lse, v_blockscale=vb if vblocks else None)
+    torch.cuda.synchronize()
+    assert device_status() == 0
+    return out, lse
+
+
+def _ungrouped(d, g):
+    q, k, v, qs, ks, vs, vb = d
+    B, SK, HK, _ = k.shape
+    spread = lambda x, dim: x.repeat_interleave(g, dim=dim).contiguous()   # noqa: E731
+    scales = spread(ks[: B * SK * HK * 4].view(B, SK, HK, 4), 2).flatten()
+    ks2 = torch.cat([scales, torch.zeros(640 * HK * g * 4, dtype=torch.uint8, device="cuda")])
+    return q, spread(k, 2), spread(v, 2), qs, ks2, vs, spread(vb, 2)
+
+
+def _exact(d, causal, vblocks):
+    q, k, v, qs, ks, vs, vb = d
+    (B, S, H, _), (_, SK, HK, _) = q.shape, k.shape
+    e4m3 = lambda x: x.view(torch.float8_e4m3fn).double()   # noqa: E731
+    scale = lambda e: torch.exp2(e.double() - 127.0)   # noqa: E731
+    qd = e4m3(q) * scale(qs[: B * S * H * 4].view(B, S, H, 4)).repeat_interleave(32, dim=3)
+    kd = e4m3(k) * scale(ks[: B * SK * HK * 4].view(B, SK, HK, 4)).repeat_interleave(32, dim=3)
+    vd = e4m3(v) * (scale(vb).repeat_interleave(32, dim=1)[:, :SK] if vblocks else vs[0].double())
+    kd, vd = (x.repeat_interleave(H // HK, dim=2) for x in (kd, vd))
+    s = torch.einsum("bihd,bjhd->bhij", qd, kd) * math.log(2.0)
+    if causal:
+        i, j = torch.arange(S, device="cuda")[:, None], torch.arange(SK, device="cuda")[None]
+        s.masked_fill_(j >= i + SK - S + 1, -math.inf)
+    return torch.einsum("bhij,bjhd->bihd", s.softmax(-1), vd), s.logsumexp(-1)
+
+
+@pytest.mark.parametrize("shape", [(2, 8, 2, 1, 700), (1, 16, 1, 3, 300), (3, 4, 2, 65, 1337), (1, 32, 2, 9, 640), (2, 8, 1, 130, 512), (1, 8, 2, 33, 129)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("option", ["plain", "causal", "vblocks", "kvsplit"])
+def test_packed_heads_give_the_bytes_of_separate_heads(shape, option):
+    from amdgpu_rustdsl_b200 import _abi
+    B, H, HK, S, SK = shape
+    d = _inputs(*shape)
+    path, splits = ("kvsplit", 2) if option == "kvsplit" else ("vs128", None)
+    got, want = (_run(x, path, splits, option == "causal", option == "vblocks", _abi.FLAG_NO_TAIL_SPLIT) for x in (d, _ungrouped(d, H // HK)))
+    assert torch.equal(got[0].view(torch.int16), want[0].view(torch.int16))
+    assert got[1] is None or torch.equal(got[1].view(torch.int32), want[1].view(torch.int32))
+
+
+# cut between 2, 4, 8 and 16 CTAs (as far as the device holds such clusters), with ragged ends, one row, full row blocks and rows past the sequence
+@pytest.mark.parametrize("shape", [(1, 8, 1, 1, 512), (1, 1, 1, 1, 32768), (2, 8, 2, 5, 8191), (1, 4, 4, 300, 4100), (1, 2, 2, 128, 16384), (8, 8, 1, 16, 3000), (1, 16, 4, 512, 2049)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("option", ["plain", "causal", "vblocks", "kvsplit"])
+def test_items_cut_between_ctas_agree_with_whole_items(shape, option):
+    from amdgpu_rustdsl_b200 import _abi
+    d = _inputs(*shape, seed=5)
+    path, splits = ("kvsplit", 2) if option == "kvsplit" else ("vs128", None)
+    (got, got_lse), (want, want_lse) = (_run(d, path, splits, option == "causal", option == "vblocks", f) for f in (0, _abi.FLAG_NO_TAIL_SPLIT))
+    ref, ref_lse = _exact(d, option == "causal", option == "vblocks")
+    err = [(x.double() - ref).norm().item() for x in (got, want)]
+    # A part's references are those of its own keys, at or below the whole item's, so no weight of P is further below its reference (and none rounds more
+    # coarsely) than uncut; the rest is the order of f32 sums. The allowance is for errors that happened to cancel in one of the two: 128 columns share
+    # a row's weights, the smallest case has 8 rows, and the norms of two sets of 8 errors differ by a quarter or so
+    assert err[0] <= 1.3 * err[1] + 2.0 ** -9 * ref.norm().item(), err
+    # a weight is off by 2^-4 from e4m3 rounding and 0.062 from the linear mantissa at most, in the sum as in the product
+    vmax = 448.0 if option == "vblocks" else 448.0 * d[5][0].item()   # (block scales up to 2^0)
+    assert (got.double() - ref).abs().max().item() <= 2 * 0.125 / (1 - 0.125) * vmax
+    if got_lse is not None:
+        assert (got_lse.double() - ref_lse).abs().max().item() <= 0.134   # -ln(1 - 0.125)
