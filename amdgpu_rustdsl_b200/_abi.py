@@ -19,6 +19,7 @@ FLAG_CAUSAL = 0x8
 FLAG_F32_PARTIALS = 0x10
 FLAG_NO_TAIL_SPLIT = 0x20
 FLAG_FUSED_COMBINE = 0x40
+FLAG_REF_TILES_SHIFT = 8
 TRACE_BYTES = 4 * (16384 + 16384 + 256 + 4096 + 2048)
 PEER_HANDLE_BYTES, PEER_MAX_GPUS, PEER_PLAN_BYTES = 64, 8, 1152
 STATIC_SCRATCH_MAX_ROW_SPLITS = 65536   # FMHA_MXFP8_STATIC_SCRATCH_MAX_ROW_SPLITS
@@ -119,6 +120,8 @@ def load():
     lib.fmha_mxfp8_grid.argtypes = [C.c_int, C.c_void_p, C.POINTER(Symbols), u32x3]
     lib.fmha_mxfp8_launch.restype = C.c_int
     lib.fmha_mxfp8_launch.argtypes = [C.c_int, C.c_void_p, u32x3, C.c_void_p]
+    lib.fmha_mxfp8_auto_unsplit.restype = C.c_int
+    lib.fmha_mxfp8_auto_unsplit.argtypes = [C.c_uint64, C.c_uint64, C.c_uint64, C.c_uint64, C.c_uint64, C.c_uint32]
     lib.fmha_mxfp8_dispatch.restype = None
     lib.fmha_mxfp8_dispatch.argtypes = [C.c_uint64, C.c_uint64, C.c_uint64, C.c_uint64, C.POINTER(C.c_int), C.POINTER(C.c_uint32)]
     lib.fmha_mxfp8_auto.restype = C.c_int
@@ -162,7 +165,7 @@ def load():
 
 EXPORTS = (
     "fmha_mxfp8_kernel_name", "fmha_mxfp8_kernarg_size", "fmha_mxfp8_workgroup_size", "fmha_mxfp8_validate", "fmha_mxfp8_grid",
-    "fmha_mxfp8_launch", "fmha_mxfp8_dispatch", "fmha_mxfp8_auto", "fmha_mxfp8_device_status", "fmha_mxfp8_trace_attach",
+    "fmha_mxfp8_launch", "fmha_mxfp8_dispatch", "fmha_mxfp8_auto_unsplit", "fmha_mxfp8_auto", "fmha_mxfp8_device_status", "fmha_mxfp8_trace_attach",
     "fmha_mxfp8_mma_issue_ceiling", "fmha_mxfp8_selftest_bounded_wait", "fmha_mxfp8_kvsplit_static_scratch", "fmha_mxfp8_quantize_qk", "fmha_mxfp8_quantize_v", "fmha_mxfp8_combine_f32", "fmha_mxfp8_peer_alloc", "fmha_mxfp8_peer_open", "fmha_mxfp8_peer_close", "fmha_mxfp8_peer_free",
     "fmha_mxfp8_peer_plan_build", "fmha_mxfp8_combine_scatter", "fmha_mxfp8_copy_async", "fmha_mxfp8_peer_barrier",
 )

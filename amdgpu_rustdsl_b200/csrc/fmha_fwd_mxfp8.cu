@@ -68,9 +68,6 @@ constexpr int kCols = 128;                  // score columns per softmax thread
 constexpr int kThreads = 32 * (4 + 8 + 4);   // 4 service warps, 8 softmax warps, 4 epilogue warps
 // The register file (64 K registers) is dealt out unevenly once the roles part: every thread starts with kMaxRegs, the service and the
 // epilogue warpgroups give most of theirs back and the two softmax warpgroups take them.
-#ifndef MXA_MIN_PART
-#define MXA_MIN_PART 2
-#endif
 #ifndef MXA_SERVICE_REGS
 #define MXA_SERVICE_REGS 56
 #define MXA_SOFTMAX_REGS 176
@@ -858,7 +855,8 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             // 2^(base - offset), in f32; only a row that grows by more than kRebase binades past its base (f32 has room for twice that) gets a
             // new base, and O and L are then rescaled in tensor memory.
             // A block's reference is the one before it (of this group's last tile, or of the other group's tile before that if that is higher), or
-            // ceil(block maximum) if the maximum passes that by more than the threshold: an integer that only grows within an item.
+            // ceil(block maximum) if the maximum passes that by more than the threshold: an integer that only grows, within an item or (ref_mask) a run of
+            // its tiles.
             // The maximum of block b + 1 is taken while block b is converted. The conversion is a software pipeline over the 32 words: word c's
             // exp2 (two values) and bit-built values (two) are started kConvDepth words before they are packed.
             auto tile_lazy = [&](int j, auto masked_c) {
@@ -866,6 +864,8 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 const uint32_t g = g0 + static_cast<uint32_t>(j);
                 const uint32_t k = g >> 1;   // this parity's tile counter
                 float* st_trace = (cta_traced && r == 0) ? p.trace : nullptr;
+                const uint32_t j_seg = static_cast<uint32_t>(j) & p.ref_mask;   // tile within its run of tiles that share a reference
+                if (j_seg < 2u) ref = -INFINITY;                                // this group's first tile of the run
                 stamp(st_trace, par, static_cast<int>(g), 0);
                 if (!mbar_wait(bar_s_full(par), k & 1u, abort_flag)) ok = false;   // no divergent exit: a failed wait only clears `ok`, the vote after the tile loop ends the role
                 tc_fence_after_sync();
@@ -991,7 +991,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         scale_o(rebase ? ex2_approx(base_prev - base) : 1.0f);
                     }
                 }
-                if (j > 0) ref = fmaxf(ref, ref_prev);
+                if (j_seg != 0u) ref = fmaxf(ref, ref_prev);
                 p_ready = true;
                 stamp(st_trace, par, static_cast<int>(g), 7);
             };
@@ -1608,7 +1608,6 @@ cudaError_t launch_attention(const CUtensorMap& tm_q, const CUtensorMap& tm_k, c
     }
     const uint32_t even_sms = static_cast<uint32_t>(sms) & ~1u;
     constexpr uint32_t kMinTilesForPairs = 48u;
-    constexpr uint32_t kMinTilesPerPart = MXA_MIN_PART;
     // how many clusters of `cluster` CTAs of kernel k the device holds at once (asked once per device, kernel and size, and kept in `known`)
     auto clusters_that_fit = [&](int k, uint32_t cluster, std::atomic<int>& known) -> uint32_t {
         int n = known.load(std::memory_order_relaxed);
@@ -1628,15 +1627,22 @@ cudaError_t launch_attention(const CUtensorMap& tm_q, const CUtensorMap& tm_k, c
         return static_cast<uint32_t>(n);
     };
     uint32_t cluster_ctas = 1u;
-    // Few items: each is cut between the CTAs of a cluster as long as the machine holds the clusters at once and every part keeps kMinTilesPerPart
-    // key tiles. The merge stays in shared memory, with f32 partials and no workspace.
+    // Few items: each is cut between the CTAs of a cluster, as far as the machine holds the clusters at once and it is worth it. The merge stays in shared
+    // memory, with f32 partials and no workspace. What it costs, in key tiles of 0.58 us (a machine with few busy SMs): the launch as clusters
+    // 8 (64 items of 4 valid rows, 16 tiles: 15.2 us whole, 15.6 us as halves; 32 tiles: 24.7 and 20.3), the exchange of 128 rows another 5 (64 items of 128 rows,
+    // 16 tiles: 15.8 and 18.2 us; 32 tiles: 25.5 and 23.3; 8 items, 16 tiles, in 16 parts: 13.9 and 13.3). Cutting only the last of several rounds this way gained
+    // 1 % at 64 tiles and lost 4 % at 16: not done.
     const bool plain = p.trace == nullptr && p.peer == nullptr && !fused && !(p.flags & (kFlagF32Partials | kFlagNoTailSplit));
     if (lazy_recipe && plain && 2u * q.n_items <= static_cast<uint32_t>(sms)) {
         uint32_t tiles = min_tiles;
         if (causal) tiles = (min(p.SK, seq_rows + (p.SK - p.S)) + kKeys - 1) / kKeys;   // the first row block's
         const int k_cut = causal ? kFirstCut + 4 : kFirstCut + (split ? 1 : 0) + (vbs ? 2 : 0);
-        uint32_t lg = 0;
-        while (lg + 1 < kCutLogs && (q.n_items << (lg + 1)) <= static_cast<uint32_t>(sms) && tiles >= (kMinTilesPerPart << (lg + 1))) ++lg;
+        const uint32_t merge_tiles = 8u + 5u * min(p.S << p.pack_shift, static_cast<uint32_t>(kRows)) / kRows;
+        uint32_t lg = 0, best = tiles;
+        for (uint32_t l = 1; l < kCutLogs && (q.n_items << l) <= static_cast<uint32_t>(sms) && (tiles >> l) > 0u; ++l) {
+            const uint32_t cost = ((tiles + (1u << l) - 1u) >> l) + merge_tiles;
+            if (cost < best) { best = cost; lg = l; }
+        }
         if (lg > 0) {
             e = ensure_attr(k_cut);
             if (e != cudaSuccess) return e;

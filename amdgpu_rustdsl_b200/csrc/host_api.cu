@@ -3,7 +3,9 @@
 #include "../../include/fmha_mxfp8_abi.h"
 #include "kernels.h"
 
+#include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -197,6 +199,14 @@ int make_partial_map(CUtensorMap* m, void* base, uint64_t seq, uint64_t heads, u
     return r == CUDA_SUCCESS ? 0 : -static_cast<int>(r);
 }
 
+// Items of 128 query rows that a launch has: the heads of a KV head packed if that gives fewer (shift: log2 of the heads per item).
+uint64_t count_items(uint64_t b, uint64_t h, uint64_t s, uint32_t gqa_shift, uint32_t* shift) {
+    const uint64_t apart = ((s + 127) / 128) * h * b, seq_rows = 128u >> (gqa_shift <= 4u ? gqa_shift : 0u);
+    const uint64_t packed = gqa_shift <= 4u ? ((s + seq_rows - 1) / seq_rows) * (h >> gqa_shift) * b : apart;
+    *shift = packed < apart ? gqa_shift : 0u;
+    return packed < apart ? packed : apart;
+}
+
 uint32_t log2_u32(uint32_t x) {
     uint32_t l = 0;
     while ((1u << l) < x) ++l;
@@ -228,6 +238,8 @@ int launch_attention_kernel(int kernel, const void* args, const uint32_t grid[3]
     p.qs_batch_stride = a->s_descale_q_Bs;
     p.ks_batch_stride = a->s_descale_k_Bs;
     p.flags = a->ext_flags;
+    const uint32_t ref_log2 = (a->ext_flags >> FMHA_MXFP8_FLAG_REF_TILES_SHIFT) & 0xFu;
+    p.ref_mask = ref_log2 == 0u ? 0xFFFFFFFFu : (1u << ref_log2) - 1u;
     // V block scales (extension): a pointer is needed, and the mask and the diagnostics have no variant with them
     if ((p.flags & FMHA_MXFP8_FLAG_V_BLOCKSCALE) && (a->ext_ptr_v_blockscale == nullptr || (p.flags & FMHA_MXFP8_FLAG_CAUSAL) || g_trace.load(std::memory_order_relaxed) != nullptr))
         return FMHA_MXFP8_E_ARG;
@@ -267,10 +279,7 @@ int launch_attention_kernel(int kernel, const void* args, const uint32_t grid[3]
     // work either way, so the heads are packed when that gives fewer items: a decode step of one row and four heads per KV head has a quarter of
     // them, a prompt whose length is a multiple of 128 as many, and those stay as they were.
     p.pack_shift = 0;
-    if (p.gqa_shift >= 1u && p.gqa_shift <= 4u && p.trace == nullptr && p.peer == nullptr && p.fused_counters == nullptr) {
-        const uint64_t seq_rows = 128u >> p.gqa_shift;
-        if ((p.S + seq_rows - 1) / seq_rows < ((static_cast<uint64_t>(p.S) + 127) / 128 << p.gqa_shift)) p.pack_shift = p.gqa_shift;
-    }
+    if (p.trace == nullptr && p.peer == nullptr && p.fused_counters == nullptr) count_items(B, p.H, p.S, p.gqa_shift, &p.pack_shift);
     const uint32_t box_heads = 1u << p.pack_shift;
     // The four tensor maps depend on nothing but the argument block (pointers, extents, strides, flags) and the packing: a call with the bytes of an
     // earlier one reuses its maps instead of encoding them again (four driver calls; a framework calls a layer with the same buffers
@@ -416,6 +425,38 @@ void fmha_mxfp8_dispatch(uint64_t b, uint64_t h, uint64_t s, uint64_t sk, int* p
     if (splits) *splits = 0;
 }
 
+int fmha_mxfp8_auto_unsplit(uint64_t b, uint64_t h, uint64_t hk, uint64_t s, uint64_t sk, uint32_t splits) {
+    if (b == 0 || h == 0 || hk == 0 || s == 0 || sk == 0 || splits < 2 || h % hk != 0) return 0;
+    const uint64_t gqa = h / hk;
+    if ((gqa & (gqa - 1)) != 0 || gqa > 16) return 0;
+    int dev = 0, n_sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n_sms < 1) {
+        (void)cudaGetLastError();
+        n_sms = 148;
+    }
+    uint32_t shift = 0;
+    const double sms = n_sms, n = static_cast<double>(count_items(b, h, s, log2_u32(static_cast<uint32_t>(gqa)), &shift)), tiles = static_cast<double>((sk + 127) / 128);
+    // us of a launch of `items` items of `len` key tiles: a start of 5.3, per round 1 for the hand-over between items, and a key tile in 0.58 on an idle machine, 0.78 on a
+    // full one, which is what launches of 8 to 222 items of 4 to 64 tiles measured; or cut between the CTAs of clusters (launch_attention)
+    const double merge = 4.6 + 2.9 * std::min(128.0, static_cast<double>(s << shift)) / 128.0;
+    auto launch_us = [&](double items, double len) {
+        auto plain = [&](double it, double l) {
+            const double rounds = std::ceil(it / sms);
+            return 5.3 + rounds + rounds * l * (0.58 + 0.2 * it / (rounds * sms));
+        };
+        double best = plain(items, len);
+        for (double parts = 2; parts <= 16 && items * parts <= sms && parts <= len; parts *= 2) best = std::min(best, plain(items * parts, std::ceil(len / parts)) + merge);
+        return best;
+    };
+    const double whole = launch_us(n, tiles);
+    // the combine: a launch, and the f16 partials written and read at 6 TB/s
+    const double split = launch_us(n * splits, std::ceil(tiles / splits)) + 3.5 + n * 128.0 * splits * 512.0 / 6.0e6;
+    if (whole >= 0.9 * split) return 0;
+    int ref_log2 = 1;   // a split's tiles, rounded down to a power of two
+    while (ref_log2 < 15 && (2ull << ref_log2) <= ((sk + 127) / 128 + splits - 1) / splits) ++ref_log2;
+    return ref_log2;
+}
+
 int fmha_mxfp8_auto(const fmha_mxfp8_problem* pr, int path, uint32_t splits, void* stream, int* path_out, uint32_t* splits_out,
                     char* err, size_t cap) {
     if (err && cap) err[0] = 0;
@@ -423,8 +464,12 @@ int fmha_mxfp8_auto(const fmha_mxfp8_problem* pr, int path, uint32_t splits, voi
     if (pr->HK == 0 || pr->H % pr->HK != 0) return fail(err, cap, FMHA_MXFP8_E_ARG, "H must be a multiple of HK");
     const uint32_t gqa = pr->H / pr->HK;
     if ((gqa & (gqa - 1)) != 0 || gqa > 16) return fail(err, cap, FMHA_MXFP8_E_ARG, "H / HK must be a power of two <= 16");
+    int unsplit = 0;   // != 0: the dispatch's split, done by the unsplit kernel with a new reference every 2^unsplit tiles
     if (path < 0) {
         fmha_mxfp8_dispatch(pr->B, pr->H, pr->S, pr->SK, &path, &splits);
+        if (path == FMHA_MXFP8_KVSPLIT && !(pr->flags & (FMHA_MXFP8_FLAG_F32_PARTIALS | FMHA_MXFP8_FLAG_NO_TAIL_SPLIT | FMHA_MXFP8_FLAG_FUSED_COMBINE |
+                                                           FMHA_MXFP8_FLAG_EXACT_REBASE)))
+            unsplit = fmha_mxfp8_auto_unsplit(pr->B, pr->H, pr->HK, pr->S, pr->SK, splits);
         if ((pr->flags & FMHA_MXFP8_FLAG_CAUSAL) && path == FMHA_MXFP8_KVSPLIT) {   // the causal extension has no split form
             path = FMHA_MXFP8_VS128;
             splits = 0;
@@ -491,6 +536,18 @@ int fmha_mxfp8_auto(const fmha_mxfp8_problem* pr, int path, uint32_t splits, voi
     fmha_mxfp8_grid(FMHA_MXFP8_COMBINE8H, &c, nullptr, cgrid);
     r = fmha_mxfp8_validate(FMHA_MXFP8_COMBINE8H, &c, &csz, cgrid, nullptr, err, cap);
     if (r) return r;
+    if (unsplit > 0) {   // (behind the split's own checks: what they refuse stays refused)
+        fmha_mxfp8_attn_args u;
+        std::memset(&u, 0, sizeof u);
+        std::memcpy(&u, &a, offsetof(fmha_mxfp8_kvsplit_args, ptr_ohat));
+        const uint32_t ugrid[3] = {static_cast<uint32_t>((S + 255) / 256), pr->H, pr->B};
+        u.ext_flags |= static_cast<uint32_t>(unsplit) << FMHA_MXFP8_FLAG_REF_TILES_SHIFT;
+        r = fmha_mxfp8_validate(FMHA_MXFP8_VS128, &u, &sz, ugrid, &sy, err, cap);
+        if (r) return r;
+        r = fmha_mxfp8_launch(FMHA_MXFP8_VS128, &u, ugrid, stream);
+        if (r) return fail(err, cap, r, "launch failed");
+        return 0;
+    }
     if (pr->flags & FMHA_MXFP8_FLAG_FUSED_COMBINE) {
         // one kernel: the counters sit behind the f16 partials in the f32-sized allocation and are cleared in front of every call
         const uint64_t n_blocks = B * H * ((S + 127) / 128), off = static_cast<uint64_t>(splits) * rows_total * 256u;

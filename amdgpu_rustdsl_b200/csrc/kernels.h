@@ -50,6 +50,8 @@ struct AttnParams {
     uint32_t qs_batch_stride, ks_batch_stride;  // bytes
     uint32_t splits, split_log2, rows_total;
     uint32_t flags;
+    // long-sequence recipe: the softmax starts from a new reference at every tile j of an item with (j & ref_mask) == 0. All ones: once per item
+    uint32_t ref_mask;
     // work decomposition of the persistent kernel, filled in by launch_attention: n_items work items (128 query rows of one (batch, head
     // [, split])); the CTAs walk work units 0 .. n_work-1. Units below tail_base are whole items. With tail_split the items of the last,
     // partly filled round are cut in two key ranges each: unit tail_base + 2 i + h is half h of item tail_base + i, and the two CTAs of a

@@ -105,6 +105,7 @@ def fmha_fwd_mxfp8(q, k, v, q_scale, k_scale, v_scale, out, *, path="auto", spli
     v_scale  f32 buffer of at least 4096 bytes, element 0 is the V descale
     out      [B, S, H, 128]  bf16
     path     "auto" | "vs128" | "t128" | "kvsplit" (splits in {2, 4, 8}).  Returns (path, splits) like the reference.
+             "auto" follows the reference's dispatch; where that says kvsplit and one unsplit launch does the work faster, that is what runs.
     fused_combine  extension: on the kvsplit path the split kernel also merges the partials (the CTA that stores a row block's last partial
              does it), so no combine kernel is launched; same bytes as the two-kernel form. Ignored on the unsplit paths. If a launch ever
              fails (``device_status() != 0``), call ``reset_workspaces()`` before the next fused call: the arrival counters may be left non-zero.
@@ -152,8 +153,11 @@ def fmha_fwd_mxfp8(q, k, v, q_scale, k_scale, v_scale, out, *, path="auto", spli
         flags |= _abi.FLAG_CAUSAL
         if SK < S:
             raise ValueError("fmha_fwd_mxfp8: causal needs SK >= S")
+    unsplit = False
     if path == "auto":
         path, splits = select_path(B, H, S, SK)
+        # the dispatch's split, where the unsplit kernel does that work faster (not where the caller chose the partials' format, whole items, the fused merge or the short recipe)
+        unsplit = path == "kvsplit" and not flags & (_abi.FLAG_F32_PARTIALS | _abi.FLAG_NO_TAIL_SPLIT | _abi.FLAG_FUSED_COMBINE | _abi.FLAG_EXACT_REBASE)
         if causal and path == "kvsplit":
             path, splits = "vs128", 0
     elif path == "kvsplit":
@@ -162,7 +166,12 @@ def fmha_fwd_mxfp8(q, k, v, q_scale, k_scale, v_scale, out, *, path="auto", spli
     # the library works on the current device (status word, SM count, kernel attributes, stream 0): make it the tensors' device
     record = []
     with torch.cuda.device(q.device):
-        ran = _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, path, splits, stream, check, flags, v_blockscale, lse, B, S, H, SK, HK, record)
+        ref_log2 = lib.fmha_mxfp8_auto_unsplit(B, H, HK, S, SK, splits) if unsplit and path == "kvsplit" else 0
+        if ref_log2:
+            _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, "vs128", 0, stream, check, flags | ref_log2 << _abi.FLAG_REF_TILES_SHIFT, v_blockscale, None, B, S, H, SK, HK, record)
+            ran = path, splits
+        else:
+            ran = _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, path, splits, stream, check, flags, v_blockscale, lse, B, S, H, SK, HK, record)
     if len(_calls) >= 256:
         _calls.clear()
     _calls[key] = (_ws_generation, record, ran)   # the key holds the stream: the split path's workspaces belong to one

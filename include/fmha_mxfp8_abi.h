@@ -78,6 +78,11 @@ enum fmha_mxfp8_error {
  * and clears them in front of every call; the bit is ignored when the path is not kvsplit.
  */
 #define FMHA_MXFP8_FLAG_FUSED_COMBINE 0x40u
+/*
+ * Bits 8 to 11, a number n: with n > 0 the long-sequence softmax of the unsplit kernels starts from a new reference every 2^n key tiles of a row block
+ * instead of once. Weights of P far below a reference lose bits; a shorter run keeps them closer to their own keys.
+ */
+#define FMHA_MXFP8_FLAG_REF_TILES_SHIFT 8
 
 #pragma pack(push, 1)
 /*
@@ -279,6 +284,13 @@ int fmha_mxfp8_launch(int kernel, const void* args, const uint32_t grid[3], void
  * mirrored in tests/gpu/ref_host.cpp:124-155). *path is FMHA_MXFP8_VS128, _T128 or _KVSPLIT; *splits is 0, 2 or 4.
  */
 void fmha_mxfp8_dispatch(uint64_t b, uint64_t h, uint64_t s, uint64_t sk, int* path, uint32_t* splits);
+/*
+ * Not 0 if, on the current device, the unsplit kernel does the work of a dispatched `splits`-way split faster than the split kernel and its combine (it cuts
+ * few row blocks between the CTAs of clusters itself, and needs no partials in memory). The default path runs it then, and still reports the
+ * dispatch's answer; a split that the caller asked for by name is always run as one. The value n is what belongs into the flags' REF_TILES field: a
+ * split's softmax starts from the split's own keys, and with a new reference every 2^n key tiles the unsplit kernel's is no further from the keys it meets.
+ */
+int fmha_mxfp8_auto_unsplit(uint64_t b, uint64_t h, uint64_t hk, uint64_t s, uint64_t sk, uint32_t splits);
 
 /* Tensors and workspaces of one forward call, all device pointers, packed BSHD as the contract demands. */
 typedef struct fmha_mxfp8_problem {
@@ -302,7 +314,7 @@ typedef struct fmha_mxfp8_problem {
  * The whole default path `fmha_fwd_hd128_mxfp8_auto`: dispatch (or a forced path), fill the Args, validate, launch (kvsplit: both
  * kernels, same stream). Mirrors python/amdgpu_jit/ops.py:88-143 (`fmha_fwd_mxfp8`) and tests/gpu/ref_host.cpp:342-397,516-569.
  * path: -1 = auto, else FMHA_MXFP8_VS128 / _T128 / _KVSPLIT; splits: used when path is _KVSPLIT (2, 4 or 8; 0 = 4).
- * On return *path_out / *splits_out (if non-NULL) hold what ran. Allocates nothing.
+ * On return *path_out / *splits_out (if non-NULL) hold the path taken, in auto the dispatch's answer (see fmha_mxfp8_auto_unsplit). Allocates nothing.
  */
 int fmha_mxfp8_auto(const fmha_mxfp8_problem* prob, int path, uint32_t splits, void* stream, int* path_out, uint32_t* splits_out,
                     char* err, size_t cap);

@@ -94,3 +94,23 @@ def test_items_cut_between_ctas_agree_with_whole_items(shape, option):
     assert (got.double() - ref).abs().max().item() <= 2 * 0.125 / (1 - 0.125) * vmax
     if got_lse is not None:
         assert (got_lse.double() - ref_lse).abs().max().item() <= 0.134   # -ln(1 - 0.125)
+
+
+@pytest.mark.parametrize("shape,ref_log2", [((1, 8, 8, 2048, 2048), 2), ((1, 8, 2, 1, 4096), 3), ((2, 4, 4, 1000, 2050), 2), ((1, 16, 4, 512, 16384), 0), ((1, 8, 2, 1, 32768), 0)], ids=lambda s: str(s).replace(" ", ""))
+def test_a_dispatched_split_runs_as_the_faster_of_the_two_forms(shape, ref_log2):
+    """The entry reports the dispatch's answer either way, and gives the bytes of the form that the rule names."""
+    from amdgpu_rustdsl_b200 import _abi, fmha_fwd_mxfp8, select_path
+    B, H, HK, S, SK = shape
+    path, splits = select_path(B, H, S, SK)
+    assert path == "kvsplit" and _abi.load().fmha_mxfp8_auto_unsplit(B, H, HK, S, SK, splits) == ref_log2
+    q, k, v, qs, ks, vs, _ = d = _inputs(*shape)
+    out = torch.full((B, S, H, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    assert fmha_fwd_mxfp8(q, k, v, qs, ks, vs, out) == (path, splits)
+    want, _ = _run(d, "vs128" if ref_log2 else path, None if ref_log2 else splits, False, False, ref_log2 << _abi.FLAG_REF_TILES_SHIFT)
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+    # No further from 64 bits than the split itself: the same weights of P but for a shorter run, and f32 partials for f16 ones. The share is for errors that
+    # cancel in one of the two; 2^-9 is the rounding of the bf16 output
+    ref, _ = _exact(d, False, False)
+    split, _ = _run(d, path, splits, False, False, 0)
+    err = [(x.double() - ref).norm().item() for x in (out, split)]
+    assert err[0] <= 1.03 * err[1] + 2.0 ** -9 * ref.norm().item(), err
