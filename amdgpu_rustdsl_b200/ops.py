@@ -184,6 +184,17 @@ def _raw_stream(torch, dev):
     return get(dev.index or 0) if get is not None else torch.cuda.current_stream(dev).cuda_stream
 
 
+def _on_device(torch, dev, stream, launch):
+    """``launch(stream handle)`` with the tensors' device current: the library works on the current device. Entering and leaving it, and building the
+    stream object, cost a few us a call, which is what a short prompt's chain of calls then waits for."""
+    if stream is None:
+        stream = _raw_stream(torch, dev)
+    if torch.cuda.current_device() == (dev.index or 0):
+        return launch(stream)
+    with torch.cuda.device(dev):
+        return launch(stream)
+
+
 def _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, path, splits, stream, check, flags, v_blockscale, lse, B, S, H, SK, HK, record=None):
     sizes = _abi.BufferSizes(ptr_q=_nbytes(q), ptr_k=_nbytes(k), ptr_v=_nbytes(v), ptr_o=_nbytes(out), ptr_q_descale=_nbytes(q_scale),
                              ptr_k_descale=_nbytes(k_scale), ptr_v_descale=_nbytes(v_scale))
@@ -247,10 +258,7 @@ def quantize_qk(x, out, out_scales, *, mul=1.0, stream=None):
         raise ValueError("quantize_qk: x must be a contiguous CUDA bf16 tensor [..., 128]")
     if out.numel() != x.numel() or out.element_size() != 1 or not out.is_contiguous() or _nbytes(out_scales) < rows * 4:
         raise ValueError("quantize_qk: out must hold one byte per element and out_scales 4 bytes per row")
-    if stream is None:
-        stream = torch.cuda.current_stream(x.device).cuda_stream
-    with torch.cuda.device(x.device):
-        rc = lib.fmha_mxfp8_quantize_qk(x.data_ptr(), rows, float(mul), out.data_ptr(), out_scales.data_ptr(), C.c_void_p(stream))
+    rc = _on_device(torch, x.device, stream, lambda raw: lib.fmha_mxfp8_quantize_qk(x.data_ptr(), rows, float(mul), out.data_ptr(), out_scales.data_ptr(), C.c_void_p(raw)))
     if rc:
         raise RuntimeError(f"fmha_mxfp8_quantize_qk failed with code {rc}")
 
@@ -263,9 +271,6 @@ def quantize_v(x, out, v_descale, *, stream=None):
         raise ValueError("quantize_v: x must be a contiguous CUDA bf16 tensor with a multiple of 8 elements")
     if out.numel() != x.numel() or out.element_size() != 1 or not out.is_contiguous() or _nbytes(v_descale) < 8:
         raise ValueError("quantize_v: out must hold one byte per element and v_descale at least 8 bytes")
-    if stream is None:
-        stream = torch.cuda.current_stream(x.device).cuda_stream
-    with torch.cuda.device(x.device):
-        rc = lib.fmha_mxfp8_quantize_v(x.data_ptr(), x.numel(), out.data_ptr(), v_descale.data_ptr(), C.c_void_p(stream))
+    rc = _on_device(torch, x.device, stream, lambda raw: lib.fmha_mxfp8_quantize_v(x.data_ptr(), x.numel(), out.data_ptr(), v_descale.data_ptr(), C.c_void_p(raw)))
     if rc:
         raise RuntimeError(f"fmha_mxfp8_quantize_v failed with code {rc}")
