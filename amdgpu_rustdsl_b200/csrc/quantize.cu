@@ -190,6 +190,9 @@ constexpr unsigned kSmallCtas = 8, kSmallThreads = 1024, kSmallVecs = 4, kSmallM
 __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThreads)
 quantize_v_small_kernel(const uint4* __restrict__ x, unsigned n_vec, uint2* __restrict__ out, float* __restrict__ descale) {
     namespace cg = cooperative_groups;
+    // A CTA's shared memory may only be written by another one once it is known to have started: every thread arrives here and waits in front of the
+    // exchange, behind the loads. (Being scheduled as one cluster does not give that order, nor does the wait for the grid before.)
+    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
     pdl_begin();
     __shared__ float part[kSmallThreads / 32];
     __shared__ float cta_amax[kSmallCtas];   // [source CTA], written by all of them
@@ -207,6 +210,7 @@ quantize_v_small_kernel(const uint4* __restrict__ x, unsigned n_vec, uint2* __re
     amax = amax_warp(amax);
     if ((threadIdx.x & 31u) == 0u) part[threadIdx.x >> 5] = amax;
     __syncthreads();
+    asm volatile("barrier.cluster.wait;" ::: "memory");
     if (threadIdx.x < 32u) {
         amax = amax_warp(part[threadIdx.x]);
         if (threadIdx.x < kSmallCtas) *cluster.map_shared_rank(&cta_amax[blockIdx.x], threadIdx.x) = amax;

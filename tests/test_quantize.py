@@ -139,3 +139,28 @@ def test_quantize_v_sizes(oracle, n_vec, scale):
         e = (torch.frexp(f.abs().amax(-1)).exponent - 1 - 8 + 127).clamp(0, 254)
         assert torch.equal(s.cpu().view(rows, 4).int(), e.int())
         assert torch.equal(y.cpu(), torch.ldexp(f, (127 - e)[..., None]).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8).view(rows, 128))
+
+
+@pytest.mark.gpu
+def test_small_v_back_to_back(oracle):
+    """The one-launch form, each launch allowed to start while the one before it runs: 64 tensors of different magnitudes and sizes on one stream without a
+    wait in between. A maximum that one CTA of a cluster misses (its neighbours write it into its shared memory) shows in its bytes and the descale."""
+    torch = pytest.importorskip("torch")
+    from amdgpu_rustdsl_b200 import quantize_v
+    g = torch.Generator().manual_seed(9)
+    sizes = [8 * n for n in (1, 1000, 8192, 8193, 20000, 32768)]
+    xs = [(torch.randn(sizes[i % 6], generator=g) * 2.0 ** (i % 11 - 5)).to(torch.bfloat16) for i in range(64)]
+    for x in xs:   # the maximum in another CTA's share each time
+        x[torch.randint(0, x.numel(), (1,), generator=g)] = 7.0 * x.float().abs().max().item()
+    dev = [x.cuda() for x in xs]
+    outs = [torch.zeros(x.numel(), dtype=torch.uint8, device="cuda") for x in xs]
+    vs = [torch.zeros(2, dtype=torch.float32, device="cuda") for _ in xs]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for x, out, v in zip(dev, outs, vs):
+            quantize_v(x, out, v)
+    torch.cuda.synchronize()
+    for x, out, v in zip(xs, outs, vs):
+        vd = (x.float().abs().max() / 448.0).item()
+        assert v[0].item() == vd
+        assert torch.equal(out.cpu(), (x.float() / vd).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8))
