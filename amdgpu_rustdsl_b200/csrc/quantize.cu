@@ -119,7 +119,7 @@ __device__ __forceinline__ float v_descale_of(float amax) { return amax > 0.0f ?
 // costs a tenth of these three instructions' rate and was what the kernel waited for.
 __device__ __forceinline__ float div_by(float x, float vd, float r) {
     const float q = __fmul_rn(x, r);
-    return __fmaf_rn(__fmaf_rn(-q, vd, x), r, q);
+    return __fmaf_rn(-__fmaf_rn(q, vd, -x), r, q);   // the residual with its sign turned: x = -0 then stays -0 (the other way round it ends as -0 + 0)
 }
 constexpr float kDivLo = 0x1p-90f, kDivHi = 0x1p100f;
 

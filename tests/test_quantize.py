@@ -107,15 +107,29 @@ def test_quantise_then_attend_passes_the_gate(oracle):
 
 def test_the_division_by_a_residual_rounds_like_a_division():
     """The device quantiser of V divides by amax / 448 with a reciprocal and one residual correction. x and amax are bf16, so their 128 x 128
-    mantissas are all there is: the corrected quotient is the correctly rounded one for each."""
+    mantissas are all there is, with either sign, and the two zeros: the corrected quotient is the correctly rounded one for each, bit for bit."""
     f32, f64 = np.float32, np.float64
-    x = (128 + np.arange(128)).astype(f32)[None, :]
+    x = (128 + np.arange(128)).astype(f32)
+    x = np.concatenate([x, -x, np.array([0.0, -0.0], f32)])[None, :]
     vd = ((128 + np.arange(128)).astype(f32) / f32(448))[:, None]
     r = f32(1) / vd
     q = x * r
-    rem = (x.astype(f64) - q.astype(f64) * vd.astype(f64)).astype(f32)   # the products of two f32 and the difference are exact in f64
-    fixed = (q.astype(f64) + rem.astype(f64) * r.astype(f64)).astype(f32)
-    assert (q != x / vd).any() and np.array_equal(fixed, x / vd)
+    rem = (q.astype(f64) * vd.astype(f64) - x.astype(f64)).astype(f32)   # the products of two f32 and the difference are exact in f64
+    fixed = (-rem.astype(f64) * r.astype(f64) + q.astype(f64)).astype(f32)
+    assert (q != x / vd).any() and np.array_equal(fixed.view(np.uint32), (x / vd).view(np.uint32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_vec", [16, 32769, 1212416])   # one launch; the general form with one and with four loads per thread
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -110])   # the divisor inside the range of the correction, and below it
+def test_quantize_v_keeps_the_sign_of_zero(n_vec, scale):
+    torch = pytest.importorskip("torch")
+    from amdgpu_rustdsl_b200 import quantize_v
+    x = torch.tensor([0.0, -0.0, 1.0, -1.0, 2.0 ** -20, -(2.0 ** -20), -0.0, 0.0]).repeat(n_vec).mul(scale).to(torch.bfloat16)
+    out, vs = torch.zeros(n_vec * 8, dtype=torch.uint8, device="cuda"), torch.zeros(2, dtype=torch.float32, device="cuda")
+    quantize_v(x.cuda(), out, vs)
+    # +-448 are the bytes 0x7E and 0xFE; 2^-20 of them are below half the smallest e4m3 step
+    assert torch.equal(out.cpu(), torch.tensor([0x00, 0x80, 0x7E, 0xFE, 0x00, 0x80, 0x80, 0x00], dtype=torch.uint8).repeat(n_vec))
 
 
 @pytest.mark.gpu
