@@ -439,7 +439,8 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             cluster_joined = true;
         }
     };
-    // nothing above touches global memory; everything below may read what the previous grid in the stream wrote
+    // nothing above touches global memory; everything below may read what the previous grid in the stream wrote (a quantiser that is still writing the
+    // scales as this grid starts, for one): by TMA or with volatile loads, never through __ldg, which the compiler may move in front of the wait
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x == 0) stamp(cta_traced ? p.trace : nullptr, 2, 30, 2);   // setup done
 
@@ -492,7 +493,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     w[i] = 0x7F7F7F7Fu;   // keys past the sequence: data is zero-filled by TMA, any finite scale does
-                    if (c.live && 32 * i < c.keys_left) w[i] = __ldg(reinterpret_cast<const uint32_t*>(c.ptr + i * row_step));
+                    ld_global_u32_if(w[i], c.ptr + i * row_step, c.live && 32 * i < c.keys_left);
                 }
                 advance(c);
                 advance(c);
@@ -505,7 +506,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     const uint32_t r = min(it.row0 + (lr >> pack_shift), p.S - 1u);   // rows past the sequence reuse the last row's scales (block3.rs:110-113)
                     const uint32_t head = it.head + (lr & ((1u << pack_shift) - 1u));
                     const size_t off = static_cast<size_t>(it.batch) * p.qs_batch_stride + (static_cast<size_t>(r) * p.H + head) * 4u;
-                    w[i] = __ldg(reinterpret_cast<const uint32_t*>(p.q_descale + off));
+                    w[i] = ld_global_u32(p.q_descale + off);
                 }
             };
             // The CTA's first copies (Q tile and first K tile, first V tile of its first item) go out before anything else of the role's set-up.
@@ -562,8 +563,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         const uint32_t nblk = (p.SK + 31u) / 32u, blk0 = static_cast<uint32_t>(key) / 32u;
 #pragma unroll
                         for (uint32_t kb = 0; kb < 4u; ++kb) {
-                            if (blk0 + kb < nblk)
-                                vsc[kb] = __ldg(reinterpret_cast<const uint32_t*>(p.v_blockscale + ((static_cast<size_t>(it.batch) * nblk + blk0 + kb) * p.HK + it.kv_head) * 128u) + lane);
+                            ld_global_u32_if(vsc[kb], p.v_blockscale + ((static_cast<size_t>(it.batch) * nblk + blk0 + kb) * p.HK + it.kv_head) * 128u + 4u * static_cast<uint32_t>(lane), blk0 + kb < nblk);
                         }
                     }
                     const bool own_scales = (g & 1u) == kPar;
@@ -1087,7 +1087,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         static_assert(128u * 512u <= kStages * kTileBytes, "the exchange area is the K ring");
         auto xch_off = [&](int c, int q4) { return static_cast<uint32_t>(c) * 128u + ((static_cast<uint32_t>(q4) ^ (r & 7u)) << 4); };
         constexpr uint32_t kEpiBar = 1u;   // named barrier of the 128 epilogue threads
-        const float vd = kVbs ? 1.0f : __ldg(p.v_descale);   // with V block scales the factors are in the MMA and there is no scalar descale
+        const float vd = kVbs ? 1.0f : __uint_as_float(ld_global_u32(p.v_descale));   // with V block scales the factors are in the MMA and there is no scalar descale
         uint32_t n = 0;
         bool ok = true;
         for (uint32_t w = blockIdx.x; w < n_items; w += stride, ++n) {

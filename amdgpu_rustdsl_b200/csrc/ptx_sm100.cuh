@@ -88,6 +88,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// ----------------------------------------------------------------------------------------------- global memory
+// A load that stays behind the griddepcontrol.wait in front of it (both are volatile). __ldg does not: it promises that nothing writes the data while the
+// grid runs, which does not hold for a grid that starts while the one before it is still writing.
+__device__ __forceinline__ uint32_t ld_global_u32(const void* p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+// the same where `live`, else v as it is. Predicated: with a branch around each of the four loads of a tile of V block scales B4 H8 S2048 took 58.0 us, so 55.6
+__device__ __forceinline__ void ld_global_u32_if(uint32_t& v, const void* p, bool live) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.global.u32 %0, [%1];\n\t}" : "+r"(v) : "l"(p), "r"(static_cast<uint32_t>(live)));
+}
+
 // ----------------------------------------------------------------------------------------------- thread-block cluster (pairs of CTAs)
 __device__ __forceinline__ uint32_t cluster_nctarank() {
     uint32_t n;

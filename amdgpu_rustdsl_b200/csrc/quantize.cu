@@ -32,10 +32,11 @@ __device__ __forceinline__ void pdl_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// A 16-byte read-once load. Volatile, so that it stays behind the wait above (a plain __ldg is an invariant load, which may move across it).
+// A 16-byte read-once load. Volatile, so that it stays behind the wait above, and not of the non-coherent kind, which is for data that nothing writes while
+// the grid runs.
 __device__ __forceinline__ uint4 ld_vec(const uint4* p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 

@@ -178,3 +178,46 @@ def test_small_v_back_to_back(oracle):
         vd = (x.float().abs().max() / 448.0).item()
         assert v[0].item() == vd
         assert torch.equal(out.cpu(), (x.float() / vd).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 8, 2, 1000, 1000), (1, 2, 2, 200, 300), (2, 8, 2, 1, 4096), (1, 4, 4, 300, 2100), (1, 8, 8, 512, 4500)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("captured", [False, True])
+def test_a_chain_of_dependent_launches_reads_what_the_one_before_wrote(shape, captured):
+    """quantise -> attend, eight times over the same operand buffers with data of another magnitude each time and no wait in between (the kernels of the chain
+    may start while the one before them runs, so a scale read too early would be the last step's), against the same calls with a wait behind each."""
+    torch = pytest.importorskip("torch")
+    from amdgpu_rustdsl_b200 import Q_PRESCALE, device_status, fmha_fwd_mxfp8, quantize_qk, quantize_v
+    B, H, HK, S, SK = shape
+    g = torch.Generator(device="cuda").manual_seed(21)
+    data = [[(torch.randn(dims, generator=g, device="cuda") * 2.0 ** e).to(torch.bfloat16) for dims, e in (((B, S, H, 128), i % 3 - 2), ((B, SK, HK, 128), -(i % 2)), ((B, SK, HK, 128), 4 - i))]
+            for i in range(8)]
+    q8, k8, v8 = (torch.empty(x.shape, dtype=torch.uint8, device="cuda") for x in data[0])
+    qs = torch.zeros(B * S * H * 4 + 512 * H * 4, dtype=torch.uint8, device="cuda")
+    ks = torch.zeros(B * SK * HK * 4 + 640 * H * 4, dtype=torch.uint8, device="cuda")
+    vs = torch.zeros(1024, dtype=torch.float32, device="cuda")
+
+    def chain(outs, wait):
+        for (q, k, v), out in zip(data, outs):
+            for call in (lambda: quantize_qk(q, q8, qs, mul=Q_PRESCALE), lambda: quantize_v(v, v8, vs), lambda: quantize_qk(k, k8, ks),
+                         lambda: fmha_fwd_mxfp8(q8, k8, v8, qs, ks, vs, out)):
+                call()
+                wait()
+
+    want, got = ([torch.zeros(B, S, H, 128, dtype=torch.bfloat16, device="cuda") for _ in data] for _ in range(2))
+    chain(want, torch.cuda.synchronize)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        chain(got, lambda: None)   # (first calls: workspaces and tensor maps)
+        torch.cuda.synchronize()
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                chain(got, lambda: None)
+        for _ in range(10):
+            for x in got:
+                x.zero_()
+            graph.replay() if captured else chain(got, lambda: None)
+            torch.cuda.synchronize()
+            assert all(torch.equal(x.view(torch.int16), y.view(torch.int16)) for x, y in zip(got, want))
+    assert device_status() == 0
