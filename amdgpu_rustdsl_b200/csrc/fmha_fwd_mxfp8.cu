@@ -101,6 +101,9 @@ constexpr float kFollowWindow = 11.0f;
 // Long sequences: O and L are in units of the row's base and a tile's P carries 2^(reference - base) as its block scale. The products stay far
 // inside f32 for 2^(8.5 + 60) x 2^8.8 (the largest e4m3 V) x 2^20 keys.
 constexpr float kRebase = 60.0f;
+// Long sequences: the reference before any key with a score above -inf has been seen. Finite, so that scores of -inf (a whole block or tile of masked keys)
+// give P = 0 and not the NaN of -inf - -inf.
+constexpr float kNoRef = -3.402823466e38f;
 constexpr uint32_t kFlagCausal = 0x8u;   // FMHA_MXFP8_FLAG_CAUSAL: selects the kCausal instantiations
 constexpr uint32_t kFlagF32Partials = 0x10u;   // FMHA_MXFP8_FLAG_F32_PARTIALS: the split kernel's partial rows are f32, not f16
 constexpr uint32_t kFlagNoTailSplit = 0x20u;   // FMHA_MXFP8_FLAG_NO_TAIL_SPLIT: never cut the last round's items in two
@@ -834,7 +837,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             }
             const bool tracing = cta_traced && n == 0;
             const bool dumping = tracing && !(p.flags & 0x4u);   // flag 0x4: time stamps only, no tile dumps
-            float ref = -INFINITY;   // the row's reference (log2 units) after the last tile this thread has seen
+            float ref = lazy ? kNoRef : -INFINITY;   // the row's reference (log2 units) after the last tile this thread has seen
             float base = -INFINITY;  // long-sequence recipe: what the row's O and L are in units of
 
             uint32_t v[128];         // the row's scores of a tile, converted in place
@@ -865,7 +868,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 const uint32_t k = g >> 1;   // this parity's tile counter
                 float* st_trace = (cta_traced && r == 0) ? p.trace : nullptr;
                 const uint32_t j_seg = static_cast<uint32_t>(j) & p.ref_mask;   // tile within its run of tiles that share a reference
-                if (j_seg < 2u) ref = -INFINITY;                                // this group's first tile of the run
+                if (j_seg < 2u) ref = kNoRef;                                   // this group's first tile of the run
                 stamp(st_trace, par, static_cast<int>(g), 0);
                 if (!mbar_wait(bar_s_full(par), k & 1u, abort_flag)) ok = false;   // no divergent exit: a failed wait only clears `ok`, the vote after the tile loop ends the role
                 tc_fence_after_sync();
@@ -896,9 +899,8 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     refs[b] = ref;
                 };
                 auto use_reference = [&](int b) {
-                    const float x = kMasked && refs[b] == -INFINITY ? 0.0f : refs[b];   // no key in sight yet (causal diagonal): every P is 0 whatever the reference
-                    sh = kPOffset - x;
-                    cf = (kPOffset + 7.0f - kFastBias - x) * 0x1p-21f;
+                    sh = kPOffset - refs[b];
+                    cf = (kPOffset + 7.0f - kFastBias - refs[b]) * 0x1p-21f;
                 };
                 constexpr int kConvDepth = 8;
                 auto conv_start = [&](int c) {
@@ -1178,7 +1180,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(ps.x), "=f"(ps.y) : "r"(smem_base + SmemLayout::xstat + cut_slot(source, ro) * 8u) : "memory");
                         return ps;
                     };
-                    // the bases are integers: the weights are exact powers of two (0 for a part without a visible key, whose base is -inf)
+                    // the bases are integers: the weights are exact powers of two (0 for a part without a visible key, whose base is kNoRef)
                     float base = -INFINITY, sum = 0.0f;
                     for (uint32_t c = 0; c < parts; ++c) base = fmaxf(base, stat(c).y);
                     for (uint32_t c = 0; c < parts; ++c) {

@@ -114,3 +114,33 @@ def test_a_dispatched_split_runs_as_the_faster_of_the_two_forms(shape, ref_log2)
     split, _ = _run(d, path, splits, False, False, 0)
     err = [(x.double() - ref).norm().item() for x in (out, split)]
     assert err[0] <= 1.03 * err[1] + 2.0 ** -9 * ref.norm().item(), err
+
+
+# keys of which 32-key blocks are masked by a bias column: the first block, the first tile, the second, the last block, two of three
+MASKS = {"block0": lambda b, n: b == 0, "tile0": lambda b, n: b < 4, "tile1": lambda b, n: (b >= 4) & (b < 8), "last": lambda b, n: b == n - 1, "most": lambda b, n: b % 3 != 1}
+
+
+@pytest.mark.parametrize("pattern", MASKS)
+@pytest.mark.parametrize("lowest", [False, True])   # scores of -inf, or of about -2^125
+@pytest.mark.parametrize("shape,option", [((1, 2, 2, 200, 1337), "plain"), ((2, 8, 2, 3, 4096), "plain"), ((1, 2, 2, 700, 1000), "causal"), ((1, 2, 1, 256, 2100), "kvsplit"), ((1, 2, 2, 300, 8300), "vblocks")],
+                         ids=lambda s: s if isinstance(s, str) else "x".join(map(str, s)))
+def test_masked_blocks_of_keys_have_no_weight(pattern, lowest, shape, option):
+    """A column of 448 in Q against -448 in K with a large scale takes a key out of the softmax, whichever blocks and tiles have no other keys."""
+    q, k, v, qs, ks, vs, vb = d = _inputs(*shape, seed=8)
+    B, H, HK, S, SK = shape
+    blocks = torch.arange(SK, device="cuda") // 32
+    masked = MASKS[pattern](blocks, int(blocks[-1]) + 1)
+    q[..., 0] = 0x7E
+    qs[: B * S * H * 4].view(B, S, H, 4)[..., 0] = 127
+    k[..., 0] = 0
+    k[:, masked, :, :32] = 0
+    k[:, masked, :, 0] = 0xFE
+    ks[: B * SK * HK * 4].view(B, SK, HK, 4)[:, masked, :, 0] = 127 + 107 if lowest else 254
+    path, splits = ("kvsplit", 2) if option == "kvsplit" else ("vs128", None)
+    got, got_lse = _run(d, path, splits, option == "causal", option == "vblocks", 0)
+    ref, ref_lse = _exact(d, option == "causal", option == "vblocks")
+    # a weight is off by 2^-4 from e4m3 rounding and 0.062 from the linear mantissa at most, in the sum as in the product
+    vmax = 448.0 if option == "vblocks" else 448.0 * vs[0].item()
+    assert torch.isfinite(got).all() and (got.double() - ref).abs().max().item() <= 2 * 0.125 / (1 - 0.125) * vmax
+    if got_lse is not None:
+        assert (got_lse.double() - ref_lse).abs().max().item() <= 0.134   # -ln(1 - 0.125)
