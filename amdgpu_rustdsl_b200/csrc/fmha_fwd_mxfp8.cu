@@ -98,9 +98,12 @@ constexpr uint32_t kTmemCols = 512;
 constexpr float kPOffset = 5.0f;
 constexpr float kLazyThreshold = 3.5f;
 constexpr float kFollowWindow = 11.0f;
-// Long sequences: O and L are in units of the row's base and a tile's P carries 2^(reference - base) as its block scale. The products stay far
-// inside f32 for 2^(8.5 + 60) x 2^8.8 (the largest e4m3 V) x 2^20 keys.
-constexpr float kRebase = 60.0f;
+// Long sequences: O and L are in units of the row's base and a tile's P carries 2^(reference - base) as its block scale, as far as this many binades
+// above the base; a row that grows further gets a new base. With a scalar V descale O holds e4m3 values: the products stay far inside f32 for 2^(8.5 + 60) x
+// 2^8.8 (the largest e4m3 V) x 2^20 keys. With V block scales O holds V as it is, which may be near the end of bf16 and f32 itself, so only 8 are
+// taken from it there; a row of normal scores grows by 4 or 5 over its first 128 keys' maximum.
+template <bool kVbs>
+constexpr float kRebase = kVbs ? 8.0f : 60.0f;
 // Long sequences: the reference before any key with a score above -inf has been seen. Finite, so that scores of -inf (a whole block or tile of masked keys)
 // give P = 0 and not the NaN of -inf - -inf.
 constexpr float kNoRef = -3.402823466e38f;
@@ -960,11 +963,11 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 float ref_prev = __uint_as_float(prev.x), base_prev = base;
                 if (j > 0) {
                     if (prev.y != g - 1u && ok && !wait_slot(ref_slot(g - 1u), g - 1u, ref_prev)) ok = false;
-                    if (ref_prev - base > kRebase) base_prev = ref_prev;
+                    if (ref_prev - base > kRebase<kVbs>) base_prev = ref_prev;
                 } else {
                     base_prev = ref;
                 }
-                base = ref - base_prev > kRebase ? ref : base_prev;
+                base = ref - base_prev > kRebase<kVbs> ? ref : base_prev;
                 const bool rebase = base != base_prev;
                 // P V of this parity's previous tile must be done before its P columns and scales are overwritten (and, observed in order,
                 // this keeps the phase parity of the other parity's barrier below unambiguous)

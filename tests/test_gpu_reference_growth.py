@@ -49,3 +49,28 @@ def test_growing_rows(oracle, pattern, shape, path, splits):
     # with 200 rows whose errors spread by 1 to 1.5 of their mean the ratio of two means is uncertain by sqrt(2) * 1 / sqrt(200) = 0.1 or so
     assert ours.mean_err <= (1.10 + 0.2) * theirs.mean_err, (ours, theirs)
     assert device_status() == 0
+
+
+@pytest.mark.parametrize("pattern", ["up", "jump", "alternate"])
+@pytest.mark.parametrize("shape,path,splits", [((1, 2, 200, 1337, 1), "vs128", None), ((2, 4, 130, 4096, 2), "vs128", None)], ids=lambda s: str(s).replace(" ", ""))
+def test_growing_rows_with_large_v(oracle, pattern, shape, path, splits):
+    """V block scales may put V anywhere in the range of bf16: what a growing row adds on top of it in the accumulators must not take it past f32."""
+    from amdgpu_rustdsl_b200 import fmha_fwd_mxfp8
+    B, H, S, SK, g = shape
+    HK = H // g
+    inp = oracle.generate("normal", B, H, S, SK, HK)
+    n, exponent = -(-SK // 128), 90
+    q, k, v, qs, ks = (torch.from_numpy(x).cuda() for x in (inp.q, inp.k, inp.v, inp.qs, inp.ks.copy()))
+    add = torch.tensor([PATTERNS[pattern](t, n) for t in range(n)], dtype=torch.uint8, device="cuda").repeat_interleave(128)[:SK]
+    ks[: B * SK * HK * 4].view(B, SK, HK, 4).add_(add[None, :, None, None])
+    vb = torch.full((B, -(-SK // 32), HK, 128), 127 + exponent, dtype=torch.uint8, device="cuda")   # |V| up to 2^98.8
+    vs = torch.ones(1024, dtype=torch.float32, device="cuda")
+    out = torch.full((B, S, H, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    fmha_fwd_mxfp8(q, k, v, qs, ks, vs, out, path=path, splits=splits, v_blockscale=vb)
+    qd = q.view(torch.float8_e4m3fn).double() * torch.exp2(qs[: B * S * H * 4].view(B, S, H, 4).double() - 127).repeat_interleave(32, 3)
+    kd = k.view(torch.float8_e4m3fn).double() * torch.exp2(ks[: B * SK * HK * 4].view(B, SK, HK, 4).double() - 127).repeat_interleave(32, 3)
+    vd = v.view(torch.float8_e4m3fn).double() * 2.0 ** exponent
+    kd, vd = (x.repeat_interleave(g, dim=2) for x in (kd, vd))
+    ref = torch.einsum("bhij,bjhd->bihd", (torch.einsum("bihd,bjhd->bhij", qd, kd) * np.log(2.0)).softmax(-1), vd)
+    # weights off by 0.125 at most, as above
+    assert torch.isfinite(out).all() and (out.double() - ref).abs().max().item() <= 0.29 * vd.abs().max().item()
