@@ -19,7 +19,7 @@ FLAG_CAUSAL = 0x8
 FLAG_F32_PARTIALS = 0x10
 FLAG_NO_TAIL_SPLIT = 0x20
 FLAG_FUSED_COMBINE = 0x40
-FLAG_REF_TILES_SHIFT = 8
+FLAG_REF_TILES_SHIFT, FLAG_REF_TILES = 8, 0xF00
 TRACE_BYTES = 4 * (16384 + 16384 + 256 + 4096 + 2048)
 PEER_HANDLE_BYTES, PEER_MAX_GPUS, PEER_PLAN_BYTES = 64, 8, 1152
 STATIC_SCRATCH_MAX_ROW_SPLITS = 65536   # FMHA_MXFP8_STATIC_SCRATCH_MAX_ROW_SPLITS

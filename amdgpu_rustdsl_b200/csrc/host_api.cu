@@ -468,7 +468,7 @@ int fmha_mxfp8_auto(const fmha_mxfp8_problem* pr, int path, uint32_t splits, voi
     if (path < 0) {
         fmha_mxfp8_dispatch(pr->B, pr->H, pr->S, pr->SK, &path, &splits);
         if (path == FMHA_MXFP8_KVSPLIT && !(pr->flags & (FMHA_MXFP8_FLAG_F32_PARTIALS | FMHA_MXFP8_FLAG_NO_TAIL_SPLIT | FMHA_MXFP8_FLAG_FUSED_COMBINE |
-                                                           FMHA_MXFP8_FLAG_EXACT_REBASE)))
+                                                           FMHA_MXFP8_FLAG_EXACT_REBASE | FMHA_MXFP8_FLAG_REF_TILES)))
             unsplit = fmha_mxfp8_auto_unsplit(pr->B, pr->H, pr->HK, pr->S, pr->SK, splits);
         if ((pr->flags & FMHA_MXFP8_FLAG_CAUSAL) && path == FMHA_MXFP8_KVSPLIT) {   // the causal extension has no split form
             path = FMHA_MXFP8_VS128;

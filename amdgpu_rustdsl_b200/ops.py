@@ -156,8 +156,9 @@ def fmha_fwd_mxfp8(q, k, v, q_scale, k_scale, v_scale, out, *, path="auto", spli
     unsplit = False
     if path == "auto":
         path, splits = select_path(B, H, S, SK)
-        # the dispatch's split, where the unsplit kernel does that work faster (not where the caller chose the partials' format, whole items, the fused merge or the short recipe)
-        unsplit = path == "kvsplit" and not flags & (_abi.FLAG_F32_PARTIALS | _abi.FLAG_NO_TAIL_SPLIT | _abi.FLAG_FUSED_COMBINE | _abi.FLAG_EXACT_REBASE)
+        # the dispatch's split, where the unsplit kernel does that work faster (not where the caller chose the partials' format, whole items, the fused merge, the
+        # short recipe or the length of a reference's run)
+        unsplit = path == "kvsplit" and not flags & (_abi.FLAG_F32_PARTIALS | _abi.FLAG_NO_TAIL_SPLIT | _abi.FLAG_FUSED_COMBINE | _abi.FLAG_EXACT_REBASE | _abi.FLAG_REF_TILES)
         if causal and path == "kvsplit":
             path, splits = "vs128", 0
     elif path == "kvsplit":

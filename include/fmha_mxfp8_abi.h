@@ -79,10 +79,12 @@ enum fmha_mxfp8_error {
  */
 #define FMHA_MXFP8_FLAG_FUSED_COMBINE 0x40u
 /*
- * Bits 8 to 11, a number n: with n > 0 the long-sequence softmax of the unsplit kernels starts from a new reference every 2^n key tiles of a row block
- * instead of once. Weights of P far below a reference lose bits; a shorter run keeps them closer to their own keys.
+ * Bits 8 to 11, a number n: with n > 0 the long-sequence softmax starts from a new reference every 2^n key tiles of a row block (or of a split's part of
+ * one) instead of once. Weights of P far below a reference lose bits; a shorter run keeps them closer to their own keys. A number that the caller sets is
+ * kept: the default path then runs a dispatched split as one.
  */
 #define FMHA_MXFP8_FLAG_REF_TILES_SHIFT 8
+#define FMHA_MXFP8_FLAG_REF_TILES 0xF00u
 
 #pragma pack(push, 1)
 /*

@@ -144,3 +144,26 @@ def test_masked_blocks_of_keys_have_no_weight(pattern, lowest, shape, option):
     assert torch.isfinite(got).all() and (got.double() - ref).abs().max().item() <= 2 * 0.125 / (1 - 0.125) * vmax
     if got_lse is not None:
         assert (got_lse.double() - ref_lse).abs().max().item() <= 0.134   # -ln(1 - 0.125)
+
+
+def test_the_callers_reference_run_is_kept_on_the_default_path():
+    """The REF_TILES field in the caller's flags: the default path does not put its own number over it, here (1) or in the C entry, and runs the split."""
+    import ctypes as C
+    from amdgpu_rustdsl_b200 import _abi, fmha_fwd_mxfp8, select_path
+    shape = B, H, HK, S, SK = 1, 8, 8, 2048, 2048
+    path, splits = select_path(B, H, S, SK)
+    lib, flags = _abi.load(), 1 << _abi.FLAG_REF_TILES_SHIFT
+    assert path == "kvsplit" and lib.fmha_mxfp8_auto_unsplit(B, H, HK, S, SK, splits) == 2
+    q, k, v, qs, ks, vs, _ = d = _inputs(*shape)
+    want, _ = _run(d, path, splits, False, False, flags)
+    out, out_c = (torch.full((B, S, H, 128), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    assert fmha_fwd_mxfp8(q, k, v, qs, ks, vs, out, flags=flags) == (path, splits)
+    ws_o, ws_l = (torch.empty(splits * B * S * H * n, dtype=torch.uint8, device="cuda") for n in (512, 4))
+    pr = _abi.Problem(B=B, H=H, HK=HK, S=S, SK=SK, q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), q_descale=qs.data_ptr(), k_descale=ks.data_ptr(), v_descale=vs.data_ptr(),
+                      out=out_c.data_ptr(), q_descale_bytes=qs.numel(), k_descale_bytes=ks.numel(), v_descale_bytes=4096, ws_ohat=ws_o.data_ptr(), ws_lse=ws_l.data_ptr(),
+                      ws_ohat_bytes=ws_o.numel(), ws_lse_bytes=ws_l.numel(), v_blockscale=None, flags=flags)
+    err = C.create_string_buffer(256)
+    assert lib.fmha_mxfp8_auto(C.byref(pr), -1, 0, None, None, None, err, 256) == 0, err.value
+    torch.cuda.synchronize()
+    for x in (out, out_c):
+        assert torch.equal(x.view(torch.int16), want.view(torch.int16))
