@@ -105,7 +105,9 @@ def fmha_fwd_mxfp8(q, k, v, q_scale, k_scale, v_scale, out, *, path="auto", spli
     v_scale  f32 buffer of at least 4096 bytes, element 0 is the V descale
     out      [B, S, H, 128]  bf16
     path     "auto" | "vs128" | "t128" | "kvsplit" (splits in {2, 4, 8}).  Returns (path, splits) like the reference.
-             "auto" follows the reference's dispatch; where that says kvsplit and one unsplit launch does the work faster, that is what runs.
+             "auto" follows the reference's dispatch and returns its answer; where that says kvsplit and one unsplit launch does the work faster
+             (``fmha_mxfp8_auto_unsplit``), that is what runs. A split that is asked for by name is always run as one.
+    lse      f32 [B, H, S], natural log-sum-exps, written by the unsplit paths only ("auto" then never picks the split).
     fused_combine  extension: on the kvsplit path the split kernel also merges the partials (the CTA that stores a row block's last partial
              does it), so no combine kernel is launched; same bytes as the two-kernel form. Ignored on the unsplit paths. If a launch ever
              fails (``device_status() != 0``), call ``reset_workspaces()`` before the next fused call: the arrival counters may be left non-zero.
@@ -160,6 +162,10 @@ def fmha_fwd_mxfp8(q, k, v, q_scale, k_scale, v_scale, out, *, path="auto", spli
         # short recipe or the length of a reference's run)
         unsplit = path == "kvsplit" and not flags & (_abi.FLAG_F32_PARTIALS | _abi.FLAG_NO_TAIL_SPLIT | _abi.FLAG_FUSED_COMBINE | _abi.FLAG_EXACT_REBASE | _abi.FLAG_REF_TILES)
         if causal and path == "kvsplit":
+            path, splits = "vs128", 0
+        elif lse is not None and path == "kvsplit":
+            if not flags & (_abi.FLAG_EXACT_REBASE | _abi.FLAG_REF_TILES):   # references as near to the keys they meet as the split's
+                flags |= max(1, min(15, (-(-(-(-SK // 128)) // splits)).bit_length() - 1)) << _abi.FLAG_REF_TILES_SHIFT
             path, splits = "vs128", 0
     elif path == "kvsplit":
         splits = splits or 4

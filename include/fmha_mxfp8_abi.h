@@ -316,7 +316,10 @@ typedef struct fmha_mxfp8_problem {
  * The whole default path `fmha_fwd_hd128_mxfp8_auto`: dispatch (or a forced path), fill the Args, validate, launch (kvsplit: both
  * kernels, same stream). Mirrors python/amdgpu_jit/ops.py:88-143 (`fmha_fwd_mxfp8`) and tests/gpu/ref_host.cpp:342-397,516-569.
  * path: -1 = auto, else FMHA_MXFP8_VS128 / _T128 / _KVSPLIT; splits: used when path is _KVSPLIT (2, 4 or 8; 0 = 4).
- * On return *path_out / *splits_out (if non-NULL) hold the path taken, in auto the dispatch's answer (see fmha_mxfp8_auto_unsplit). Allocates nothing.
+ * On return *path_out / *splits_out (if non-NULL) hold the path taken, in auto the dispatch's answer: where that is kvsplit, the unsplit kernel may have done the
+ * work (it has if fmha_mxfp8_auto_unsplit says so for these sizes on this device and none of the flags F32_PARTIALS, NO_TAIL_SPLIT, FUSED_COMBINE,
+ * EXACT_REBASE and REF_TILES is set). The workspaces are scratch and must be there either way, but hold partials only after a split that was
+ * asked for by name. Allocates nothing.
  */
 int fmha_mxfp8_auto(const fmha_mxfp8_problem* prob, int path, uint32_t splits, void* stream, int* path_out, uint32_t* splits_out,
                     char* err, size_t cap);

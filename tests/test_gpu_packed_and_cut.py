@@ -167,3 +167,22 @@ def test_the_callers_reference_run_is_kept_on_the_default_path():
     torch.cuda.synchronize()
     for x in (out, out_c):
         assert torch.equal(x.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("shape", [(1, 8, 8, 2048, 2048), (1, 16, 4, 512, 16384), (1, 8, 2, 1, 32768)], ids=lambda s: "x".join(map(str, s)))
+def test_the_default_path_writes_the_log_sum_exps_it_is_asked_for(shape):
+    """Shapes that the dispatch splits (one that runs unsplit anyway, two that do not): the split has no such output, so an unsplit kernel runs and is reported."""
+    from amdgpu_rustdsl_b200 import fmha_fwd_mxfp8, select_path
+    B, H, HK, S, SK = shape
+    path, splits = select_path(B, H, S, SK)
+    assert path == "kvsplit"
+    q, k, v, qs, ks, vs, _ = d = _inputs(*shape)
+    out = torch.full((B, S, H, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    lse = torch.full((B, H, S), float("nan"), device="cuda")
+    assert fmha_fwd_mxfp8(q, k, v, qs, ks, vs, out, lse=lse) == ("vs128", 0)
+    ref, ref_lse = _exact(d, False, False)
+    assert (lse.double() - ref_lse).abs().max().item() <= 0.134   # -ln(1 - 0.125): weights off by 0.125 at most
+    # no further from 64 bits than the split (the same weights of P but for a shorter run; the allowances of the test above)
+    split, _ = _run(d, path, splits, False, False, 0)
+    err = [(x.double() - ref).norm().item() for x in (out, split)]
+    assert err[0] <= 1.03 * err[1] + 2.0 ** -9 * ref.norm().item(), err
