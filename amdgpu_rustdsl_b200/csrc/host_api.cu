@@ -213,6 +213,22 @@ uint32_t log2_u32(uint32_t x) {
     return l;
 }
 
+// SMs of the current device (asked once per device), or a B200's where there is none
+int current_sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+        n = known[dev].load(std::memory_order_relaxed);
+        if (n > 0) return n;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0) {
+            known[dev].store(n, std::memory_order_relaxed);
+            return n;
+        }
+    }
+    (void)cudaGetLastError();
+    return 148;
+}
+
 std::atomic<float*> g_trace{nullptr};
 
 int launch_attention_kernel(int kernel, const void* args, const uint32_t grid[3], cudaStream_t stream) {
@@ -429,11 +445,7 @@ int fmha_mxfp8_auto_unsplit(uint64_t b, uint64_t h, uint64_t hk, uint64_t s, uin
     if (b == 0 || h == 0 || hk == 0 || s == 0 || sk == 0 || splits < 2 || h % hk != 0) return 0;
     const uint64_t gqa = h / hk;
     if ((gqa & (gqa - 1)) != 0 || gqa > 16) return 0;
-    int dev = 0, n_sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n_sms < 1) {
-        (void)cudaGetLastError();
-        n_sms = 148;
-    }
+    const int n_sms = current_sm_count();
     uint32_t shift = 0;
     const double sms = n_sms, n = static_cast<double>(count_items(b, h, s, log2_u32(static_cast<uint32_t>(gqa)), &shift)), tiles = static_cast<double>((sk + 127) / 128);
     // us of a launch of `items` items of `len` key tiles: a start of 5.3, per round 1 for the hand-over between items, and a key tile in 0.58 on an idle machine, 0.78 on a

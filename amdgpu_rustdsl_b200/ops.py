@@ -68,9 +68,11 @@ def _check_launch(lib, kernel, args, sizes, grid, syms, stream, check, record=No
     if record is not None:
         record.append((kernel, args, grid))
     if check:
-        err = C.create_string_buffer(256)
-        rc = lib.fmha_mxfp8_validate(kernel, C.byref(args), C.byref(sizes), grid, C.byref(syms) if syms is not None else None, err, 256)
-        if rc:
+        syms = C.byref(syms) if syms is not None else None
+        rc = lib.fmha_mxfp8_validate(kernel, C.byref(args), C.byref(sizes), grid, syms, None, 0)
+        if rc:   # the message is asked for only then
+            err = C.create_string_buffer(256)
+            lib.fmha_mxfp8_validate(kernel, C.byref(args), C.byref(sizes), grid, syms, err, 256)
             raise ContractError(rc, err.value.decode())
     rc = lib.fmha_mxfp8_launch(kernel, C.byref(args), grid, C.c_void_p(stream))
     if rc:
@@ -169,16 +171,16 @@ def fmha_fwd_mxfp8(q, k, v, q_scale, k_scale, v_scale, out, *, path="auto", spli
             path, splits = "vs128", 0
     elif path == "kvsplit":
         splits = splits or 4
-    stream = raw_stream
-    # the library works on the current device (status word, SM count, kernel attributes, stream 0): make it the tensors' device
     record = []
-    with torch.cuda.device(q.device):
+
+    def launch(stream):
         ref_log2 = lib.fmha_mxfp8_auto_unsplit(B, H, HK, S, SK, splits) if unsplit and path == "kvsplit" else 0
         if ref_log2:
             _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, "vs128", 0, stream, check, flags | ref_log2 << _abi.FLAG_REF_TILES_SHIFT, v_blockscale, None, B, S, H, SK, HK, record)
-            ran = path, splits
-        else:
-            ran = _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, path, splits, stream, check, flags, v_blockscale, lse, B, S, H, SK, HK, record)
+            return path, splits
+        return _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, path, splits, stream, check, flags, v_blockscale, lse, B, S, H, SK, HK, record)
+
+    ran = _on_device(torch, dev, raw_stream, launch)
     if len(_calls) >= 256:
         _calls.clear()
     _calls[key] = (_ws_generation, record, ran)   # the key holds the stream: the split path's workspaces belong to one
@@ -192,7 +194,7 @@ def _raw_stream(torch, dev):
 
 
 def _on_device(torch, dev, stream, launch):
-    """``launch(stream handle)`` with the tensors' device current: the library works on the current device. Entering and leaving it, and building the
+    """``launch(stream handle)`` with the tensors' device current: the library works on the current device (status word, SM count, kernel attributes, stream 0). Entering and leaving it, and building the
     stream object, cost a few us a call, which is what a short prompt's chain of calls then waits for."""
     if stream is None:
         stream = _raw_stream(torch, dev)
