@@ -85,10 +85,12 @@ def test_items_cut_between_ctas_agree_with_whole_items(shape, option):
     (got, got_lse), (want, want_lse) = (_run(d, path, splits, option == "causal", option == "vblocks", f) for f in (0, _abi.FLAG_NO_TAIL_SPLIT))
     ref, ref_lse = _exact(d, option == "causal", option == "vblocks")
     err = [(x.double() - ref).norm().item() for x in (got, want)]
-    # A part's references are those of its own keys, at or below the whole item's, so no weight of P is further below its reference (and none rounds more
-    # coarsely) than uncut; the rest is the order of f32 sums. The allowance is for errors that happened to cancel in one of the two: 128 columns share
-    # a row's weights, the smallest case has 8 rows, and the norms of two sets of 8 errors differ by a quarter or so
-    assert err[0] <= 1.3 * err[1] + 2.0 ** -9 * ref.norm().item(), err
+    # A part's references start from its own keys, where the whole item's start from its first: on average no weight of P is further below its reference, and
+    # measured the parts' error is 0.64 to 1.00 of the whole items'. A single row's reference may sit up to 3.5 binades higher in a part than in the
+    # item, and its keys far below it then round more coarsely: the allowance for that is 0.3 of a row's error, which averages out over B H S rows. The other
+    # share is the rounding of the bf16 output
+    rows = shape[0] * shape[1] * shape[3]
+    assert err[0] <= (1 + 0.3 / math.sqrt(rows)) * err[1] + 2.0 ** -9 * ref.norm().item(), err
     # a weight is off by 2^-4 from e4m3 rounding and 0.062 from the linear mantissa at most, in the sum as in the product
     vmax = 448.0 if option == "vblocks" else 448.0 * d[5][0].item()   # (block scales up to 2^0)
     assert (got.double() - ref).abs().max().item() <= 2 * 0.125 / (1 - 0.125) * vmax

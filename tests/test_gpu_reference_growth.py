@@ -45,9 +45,9 @@ def test_growing_rows(oracle, pattern, shape, path, splits):
     # w(1 + d), |d| <= 0.125, an output moves by at most 2 * 0.125 / (1 - 0.125) of the largest |v| of its column
     bound = 0.29 * float(np.abs(oracle.e4m3_table()[inp.v]).max()) * inp.vdescale
     assert ours.worst_err <= bound, (ours, theirs)
-    # The gate's 1.10 on the mean, and two standard errors of it: a few keys carry such a row, so its 128 errors are one or two roundings of P, and
-    # with 200 rows whose errors spread by 1 to 1.5 of their mean the ratio of two means is uncertain by sqrt(2) * 1 / sqrt(200) = 0.1 or so
-    assert ours.mean_err <= (1.10 + 0.2) * theirs.mean_err, (ours, theirs)
+    # The gate's 1.10 on the mean, and one standard error of a ratio of two means of S rows: a few keys carry such a row, so its 128 errors are one or two
+    # roundings of P that spread by about their mean, and the ratio is uncertain by sqrt(2 / S) = 0.09 to 0.1. Measured: 0.50 to 1.10, most of them under 1
+    assert ours.mean_err <= (1.10 + (2 / S) ** 0.5) * theirs.mean_err, (ours, theirs)
     assert device_status() == 0
 
 
