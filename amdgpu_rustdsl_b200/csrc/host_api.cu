@@ -448,8 +448,10 @@ int fmha_mxfp8_auto_unsplit(uint64_t b, uint64_t h, uint64_t hk, uint64_t s, uin
     const int n_sms = current_sm_count();
     uint32_t shift = 0;
     const double sms = n_sms, n = static_cast<double>(count_items(b, h, s, log2_u32(static_cast<uint32_t>(gqa)), &shift)), tiles = static_cast<double>((sk + 127) / 128);
-    // us of a launch of `items` items of `len` key tiles: a start of 5.3, per round 1 for the hand-over between items, and a key tile in 0.58 on an idle machine, 0.78 on a
-    // full one, which is what launches of 8 to 222 items of 4 to 64 tiles measured; or cut between the CTAs of clusters (launch_attention)
+    // us of a launch of `items` items of `len` key tiles: a start of 5.3, per round 1 for the hand-over between items, and a key tile in 0.58 with few SMs busy, 0.78 with
+    // all of them, which is what launches of 8 to 222 items of 4 to 64 tiles measured; or cut between the CTAs of clusters (launch_attention). The
+    // difference is the clock, not contention: a tile is 1090 to 1180 clocks with 1 to 148 items, but under the power cap all SMs together run at 1515 to 1600
+    // MHz and a few at 1965. Where a box has another cap the two sides shift together; the margin of 10 % below is for that.
     const double merge = 4.6 + 2.9 * std::min(128.0, static_cast<double>(s << shift)) / 128.0;
     auto launch_us = [&](double items, double len) {
         auto plain = [&](double it, double l) {
