@@ -172,15 +172,13 @@ def fmha_fwd_mxfp8(q, k, v, q_scale, k_scale, v_scale, out, *, path="auto", spli
     elif path == "kvsplit":
         splits = splits or 4
     record = []
-
-    def launch(stream):
-        ref_log2 = lib.fmha_mxfp8_auto_unsplit(B, H, HK, S, SK, splits) if unsplit and path == "kvsplit" else 0
-        if ref_log2:
-            _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, "vs128", 0, stream, check, flags | ref_log2 << _abi.FLAG_REF_TILES_SHIFT, v_blockscale, None, B, S, H, SK, HK, record)
-            return path, splits
-        return _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, path, splits, stream, check, flags, v_blockscale, lse, B, S, H, SK, HK, record)
-
-    ran = _on_device(torch, dev, raw_stream, launch)
+    args = (lib, q, k, v, q_scale, k_scale, v_scale, out, path, splits, raw_stream, check, flags, v_blockscale, lse, B, S, H, SK, HK, record)
+    # (no function is defined in here for _on_device: what it would refer to could not be plain locals, which cost a remembered call 0.7 us)
+    if torch.cuda.current_device() == (dev.index or 0):
+        ran = _launch_dispatched(unsplit and path == "kvsplit", *args)
+    else:
+        with torch.cuda.device(dev):
+            ran = _launch_dispatched(unsplit and path == "kvsplit", *args)
     if len(_calls) >= 256:
         _calls.clear()
     _calls[key] = (_ws_generation, record, ran)   # the key holds the stream: the split path's workspaces belong to one
@@ -194,14 +192,23 @@ def _raw_stream(torch, dev):
 
 
 def _on_device(torch, dev, stream, launch):
-    """``launch(stream handle)`` with the tensors' device current: the library works on the current device (status word, SM count, kernel attributes, stream 0). Entering and leaving it, and building the
-    stream object, cost a few us a call, which is what a short prompt's chain of calls then waits for."""
+    """``launch(stream handle)`` with the tensors' device current: the library works on the current device (status word, SM count, kernel attributes, stream 0).
+    Entering and leaving it, and building the stream object, cost a few us a call, which is what a short prompt's chain of calls then waits for."""
     if stream is None:
         stream = _raw_stream(torch, dev)
     if torch.cuda.current_device() == (dev.index or 0):
         return launch(stream)
     with torch.cuda.device(dev):
         return launch(stream)
+
+
+def _launch_dispatched(unsplit, lib, q, k, v, q_scale, k_scale, v_scale, out, path, splits, stream, check, flags, v_blockscale, lse, B, S, H, SK, HK, record):
+    """``_launch_path``, or with ``unsplit`` the unsplit kernel in place of a dispatched split that it is faster than (the answer is the dispatch's)."""
+    ref_log2 = lib.fmha_mxfp8_auto_unsplit(B, H, HK, S, SK, splits) if unsplit else 0
+    if not ref_log2:
+        return _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, path, splits, stream, check, flags, v_blockscale, lse, B, S, H, SK, HK, record)
+    _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, "vs128", 0, stream, check, flags | ref_log2 << _abi.FLAG_REF_TILES_SHIFT, v_blockscale, None, B, S, H, SK, HK, record)
+    return path, splits
 
 
 def _launch_path(lib, q, k, v, q_scale, k_scale, v_scale, out, path, splits, stream, check, flags, v_blockscale, lse, B, S, H, SK, HK, record=None):
