@@ -19,15 +19,14 @@
 //   warp  0    Q K^T issuer: S[g % 2] = Q K_g^T as kind::mxf8f6f4.block_scale tcgen05.mma, both operands in swizzled shared memory,
 //              the E8M0 factors copied to TMEM with tcgen05.cp. Two score tiles are always ahead of the softmax.
 //   warp  1    Q / K producer: TMA loads of the Q tile (double buffered across items) and of the K ring, plus the 4-byte-per-row scale
-//              gathers (Q, and K for the tiles with an even counter), which a TMA box cannot express, written in the 32x16-byte
-//              layout tcgen05.cp expects.
+//              bytes of both, which a TMA box cannot express: 4-byte asynchronous copies straight into the 32x16-byte layout tcgen05.cp
+//              expects, arriving on the tile's barrier.
 //   warp  2    P V issuer: O += P_g V_g with P from TMEM and V (keys x head dim, i.e. MN-major B) from shared memory. The B operand
 //              is 144 wide: 128 head dims plus 16 columns of a tile of e4m3 ones, so that O[:, 128..143] (= the L columns) holds the
 //              row sums of the *quantised* P at no ALU cost (the reference sums P with a matrix instruction too, reduce.rs:163-173).
 //              It has a thread of its own: the tensor pipe takes MMAs from one thread at its full rate, but a thread that shares its
 //              scheduler with softmax warps only gets an instruction in every few clocks.
-//   warp  3    V producer: TMA loads of the V ring (K is freed after Q K^T, V after P V, so the two rings run apart), and the K scale
-//              gathers of the tiles with an odd counter.
+//   warp  3    V producer: TMA loads of the V ring (K is freed after Q K^T, V after P V, so the two rings run apart).
 //   warps 4-11 softmax, two warpgroups: warpgroup p works on the tiles with counter g = p (mod 2). Thread r of a group owns query row
 //              r = TMEM lane r: it reads the row's 128 scores from tensor memory and hands the S buffer back at once, converts block by
 //              block of 32 keys with the block's own reference, writes P (packed e4m3) with tcgen05.st and, when they change, the
@@ -390,7 +389,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     if (threadIdx.x == 0) {
         *abort_flag = 0u;
         for (int b = 0; b < 2; ++b) {
-            mbar_init(bar_q_full(b), 2);   // the TMA's expect-tx arrive + the arrive that follows the scale bytes
+            mbar_init(bar_q_full(b), 1 + 32);   // the TMA's expect-tx arrive + the producer lanes' scale copies
             mbar_init(bar_q_empty(b), 1);
             mbar_init(bar_s_full(b), 1);
             mbar_init(bar_s_free(b), kRows);
@@ -398,7 +397,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             mbar_init(bar_o_done(b), 1);
         }
         for (int st = 0; st < kStages; ++st) {
-            mbar_init(bar_k_full(st), 2);
+            mbar_init(bar_k_full(st), 1 + 32);
             mbar_init(bar_k_empty(st), 1);
             mbar_init(bar_v_full(st), kVbs ? 2 : 1);   // with V block scales: the TMA's expect-tx arrive + the arrive that follows the scale bytes
             mbar_init(bar_v_empty(st), 1);
@@ -460,61 +459,26 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kServiceRegs));
     if (warp == kKProducerWarp || warp == kVProducerWarp) {
         // =========================================================== producers: Q, K, V tiles; Q and K scales ===========================================================
-        // Warp 1 issues the Q and K tile copies and gathers the Q scales, warp 3 issues the V tile copies. The K scale bytes (4 per key,
-        // strided by the head count, which a TMA box cannot express) are gathered by both: warp 1 takes the tiles with an even counter,
-        // warp 3 the odd ones, so that neither warp's per-tile instruction stream is long (a producer that needs more clocks per tile
-        // than the softmax sets the pace of the whole CTA). A tile's scales are loaded four tiles (two of the warp's own) ahead into
-        // one of two register sets, each use naming its set statically, so that a tile never waits for loads issued behind it. The
-        // scale cursor therefore walks the items on its own.
+        // Warp 1 issues the Q and K tile copies and, with 4-byte asynchronous copies, their scale bytes (4 per row, strided by the head count, which a
+        // TMA box cannot express); warp 3 issues the V tile copies. Both run ahead as far as their rings go. The scales used to be loaded into registers four
+        // tiles ahead and stored by the two warps in turn: a K tile's scales then waited for the V ring on every second tile, and a launch's first tile for
+        // the loads of the first five (B1 H37 S512 Skv2048, 148 items of 16 tiles: 16.3 us, so 15.2; B4 H8 S2048 48.7, so 47.7).
         auto producer = [&](auto is_k_c) {
             constexpr bool kIsK = decltype(is_k_c)::value;
-            constexpr uint32_t kPar = kIsK ? 0u : 1u;   // parity of the tile counters whose K scales this warp gathers
-            const uint32_t row_step = 32u * p.HK * 4u, tile_step = 4u * row_step;   // bytes between a lane's four keys / between key tiles
-            struct ScaleCursor {
-                const uint8_t* ptr;   // scale word of this lane's first key of the tile
-                int keys_left;        // sequence keys from the tile's first key on (lanes compare against it)
-                int tiles_left;       // of the item
-                uint32_t w;           // the item
-                bool live;
-            };
-            auto enter_item = [&](ScaleCursor& c) {
-                c.live = c.w < n_items;
-                if (!c.live) return;
-                const Item it = decode_item<kSplit, kCausal, kCluster, kPack>(c.w, p);
-                c.ptr = p.k_descale + static_cast<size_t>(it.batch) * p.ks_batch_stride + (static_cast<size_t>(it.key_lo + lane) * p.HK + it.kv_head) * 4u;
-                c.keys_left = static_cast<int>(p.SK - it.key_lo) - lane;
-                c.tiles_left = it.n_tiles;
-            };
-            auto advance = [&](ScaleCursor& c) {
-                if (!c.live) return;
-                c.ptr += tile_step;
-                c.keys_left -= kKeys;
-                if (--c.tiles_left == 0) {
-                    c.w += stride;
-                    enter_item(c);
-                }
-            };
-            // loads the scales of the cursor's tile and moves the cursor to the warp's next tile (two on)
-            auto load_and_advance = [&](ScaleCursor& c, uint32_t (&w)[4]) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    w[i] = 0x7F7F7F7Fu;   // keys past the sequence: data is zero-filled by TMA, any finite scale does
-                    ld_global_u32_if(w[i], c.ptr + i * row_step, c.live && 32 * i < c.keys_left);
-                }
-                advance(c);
-                advance(c);
-            };
-            // Q scale bytes -> [row % 32][row / 32][4] (the layout tcgen05.cp 32x128b.warpx4 spreads over the four lane quadrants)
-            auto load_q_scales = [&](const Item& it, uint32_t (&w)[4]) {
+            // E8M0 words of 128 rows -> [row % 32][row / 32][4] (the layout tcgen05.cp 32x128b.warpx4 spreads over the four lane quadrants): lane l copies
+            // rows l, l + 32, ... The copies arrive on the tile's barrier when they have landed (32 arrivals).
+            auto copy_q_scales = [&](const Item& it, uint32_t qb) {
+                const uint32_t dst = sfq_smem + qb * kSfBytes + static_cast<uint32_t>(lane) * 16u;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const uint32_t lr = lane + 32 * i;
                     const uint32_t r = min(it.row0 + (lr >> pack_shift), p.S - 1u);   // rows past the sequence reuse the last row's scales (block3.rs:110-113)
                     const uint32_t head = it.head + (lr & ((1u << pack_shift) - 1u));
-                    const size_t off = static_cast<size_t>(it.batch) * p.qs_batch_stride + (static_cast<size_t>(r) * p.H + head) * 4u;
-                    w[i] = ld_global_u32(p.q_descale + off);
+                    cp_async_4(dst + 4u * i, p.q_descale + static_cast<size_t>(it.batch) * p.qs_batch_stride + (static_cast<size_t>(r) * p.H + head) * 4u, 4u);
                 }
+                cp_async_arrive(bar_q_full(qb));
             };
+            const uint32_t row_step = 32u * p.HK * 4u, tile_step = 4u * row_step;   // of the K scales: bytes between a lane's four keys / between key tiles
             // The CTA's first copies (Q tile and first K tile, first V tile of its first item) go out before anything else of the role's set-up.
             if (blockIdx.x < n_items && elect_one_sync()) {
                 const Item it = decode_item<kSplit, kCausal, kCluster, kPack>(blockIdx.x, p);
@@ -530,15 +494,6 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     tma_load_4d(v_smem, &tm_v, bar_v_full(0), 0, static_cast<int>(it.kv_head), static_cast<int>(it.key_lo), static_cast<int>(it.batch));
                 }
             }
-            ScaleCursor cs;
-            cs.w = blockIdx.x;
-            enter_item(cs);
-            if (kPar) advance(cs);   // this warp's first tile is the CTA's second
-            uint32_t wq[4] = {0u, 0u, 0u, 0u}, w0[4], w1[4];
-            if (kIsK && blockIdx.x < n_items) load_q_scales(decode_item<kSplit, kCausal, kCluster, kPack>(blockIdx.x, p), wq);
-            load_and_advance(cs, w0);
-            load_and_advance(cs, w1);
-
             uint32_t g = 0, n = 0, ph = 0, q_issued = 0;   // g: the running tile counter
             int st = 0;
             bool ok = true;
@@ -549,18 +504,16 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     // the Q buffer was last used two items ago
                     if (n >= 2) ok = mbar_wait(bar_q_empty(qb), ((n >> 1) - 1u) & 1u, abort_flag);
                     if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
-                    // the tile copy goes out first: it does not depend on the scale bytes, whose global loads may still be in flight
                     if (n > 0 && elect_one_sync()) {
                         mbar_arrive_expect_tx(bar_q_full(qb), kTileBytes);
                         tma_load_4d(q_smem + qb * kTileBytes, &tm_q, bar_q_full(qb), 0, static_cast<int>(it.head), static_cast<int>(it.row0), static_cast<int>(it.batch));
                     }
-                    *reinterpret_cast<uint4*>(smem_gen + SmemLayout::sfq + qb * kSfBytes + lane * 16) = make_uint4(wq[0], wq[1], wq[2], wq[3]);
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (elect_one_sync()) mbar_arrive(bar_q_full(qb));
+                    copy_q_scales(it, qb);
                     ++q_issued;
-                    if (w + stride < n_items) load_q_scales(decode_item<kSplit, kCausal, kCluster, kPack>(w + stride, p), wq);   // the next item's Q scales, a whole item ahead
                 }
+                // scale word of this lane's first key of the tile; sequence keys from the tile's first key on (lanes compare against it)
+                const uint8_t* k_scales = p.k_descale + static_cast<size_t>(it.batch) * p.ks_batch_stride + (static_cast<size_t>(it.key_lo + lane) * p.HK + it.kv_head) * 4u;
+                int keys_left = static_cast<int>(p.SK - it.key_lo) - lane;
                 float* k_trace = cta_traced ? p.trace : nullptr;   // stamps are indexed by the running tile counter
                 int key = static_cast<int>(it.key_lo);
                 for (int j = 0; j < it.n_tiles; ++j, key += kKeys) {
@@ -572,25 +525,21 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             ld_global_u32_if(vsc[kb], p.v_blockscale + ((static_cast<size_t>(it.batch) * nblk + blk0 + kb) * p.HK + it.kv_head) * 128u + 4u * static_cast<uint32_t>(lane), blk0 + kb < nblk);
                         }
                     }
-                    const bool own_scales = (g & 1u) == kPar;
                     // K: the stage (tile and scale bytes) is free once Q K^T of the tile that held it is done
-                    if ((kIsK || own_scales) && g >= static_cast<uint32_t>(kStages)) ok = mbar_wait(bar_k_empty(st), ph ^ 1u, abort_flag);
-                    if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
-                    if (kIsK && g > 0 && elect_one_sync()) {
-                        stamp(k_trace, 2, static_cast<int>(g), 6);
-                        mbar_arrive_expect_tx(bar_k_full(st), kTileBytes);
-                        tma_load_4d(k_smem + st * kTileBytes, &tm_k, bar_k_full(st), 0, static_cast<int>(it.kv_head), key, static_cast<int>(it.batch));
-                    }
-                    if (own_scales) {
-                        uint4* sf_dst = reinterpret_cast<uint4*>(smem_gen + SmemLayout::sfk + st * kSfBytes + lane * 16);
-                        auto put_and_refill = [&](uint32_t (&set)[4]) {
-                            *sf_dst = make_uint4(set[0], set[1], set[2], set[3]);
-                            load_and_advance(cs, set);   // for the tile four ahead
-                        };
-                        if (g & 2u) put_and_refill(w1); else put_and_refill(w0);
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (elect_one_sync()) mbar_arrive(bar_k_full(st));
+                    if (kIsK) {
+                        if (g >= static_cast<uint32_t>(kStages)) ok = mbar_wait(bar_k_empty(st), ph ^ 1u, abort_flag);
+                        if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
+                        if (g > 0 && elect_one_sync()) {
+                            stamp(k_trace, 2, static_cast<int>(g), 6);
+                            mbar_arrive_expect_tx(bar_k_full(st), kTileBytes);
+                            tma_load_4d(k_smem + st * kTileBytes, &tm_k, bar_k_full(st), 0, static_cast<int>(it.kv_head), key, static_cast<int>(it.batch));
+                        }
+                        const uint32_t dst = sfk_smem + static_cast<uint32_t>(st) * kSfBytes + static_cast<uint32_t>(lane) * 16u;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) cp_async_4(dst + 4u * i, k_scales + i * row_step, 32 * i < keys_left ? 4u : 0u);   // (keys past the sequence: zeros; their data is zero-filled too)
+                        cp_async_arrive(bar_k_full(st));
+                        k_scales += tile_step;
+                        keys_left -= kKeys;
                     }
                     if (!kIsK) {
                         // V: the stage is free once P V of the tile that held it is done
@@ -624,8 +573,9 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     if (++st == kStages) { st = 0; ph ^= 1u; }
                 }
             }
+            cp_async_wait_all();
             if (*abort_flag != 0u) {
-                // leaving early: let the copies already in flight land before the CTA's shared memory is given back
+                // leaving early: let the tile copies already in flight land before the CTA's shared memory is given back
                 for (uint32_t t = g > static_cast<uint32_t>(kStages) ? g - kStages : 0u; t < g; ++t) {
                     const long long t0 = clock64();
                     while (!mbar_test_wait(kIsK ? bar_k_full(t % kStages) : bar_v_full(t % kStages), (t / kStages) & 1u) && clock64() - t0 < kWaitBudgetCycles) {}
@@ -671,6 +621,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 ok = mbar_wait(bar_q_full(qb), (n >> 1) & 1u, abort_flag);
                 if (!ok) break;
                 tc_fence_after_sync();
+                fence_proxy_async_smem();   // the scale bytes are written by the producer lanes' asynchronous copies (generic writes, acquired by the wait) and read by tcgen05.cp
                 // issued behind the previous item's MMAs by the same thread, so it cannot overtake their reads of these columns
                 if (elect_one_sync()) tmem_cp_sf(t_sfq, dsfq0 + static_cast<uint64_t>((qb * kSfBytes) >> 4));
                 const uint64_t dq = dq0 + static_cast<uint64_t>((qb * kTileBytes) >> 4);
@@ -679,6 +630,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     ok = mbar_wait(bar_k_full(st), ph, abort_flag);
                     if (ok && g >= 2) ok = mbar_wait(bar_s_free(g & 1u), ((g >> 1) - 1u) & 1u, abort_flag);
                     if (!ok) break;
+                    fence_proxy_async_smem();   // (the K scales' copies are generic writes too)
                     tc_fence_after_sync();
                     if (lane == 0) stamp(mma_trace, 2, static_cast<int>(g), 2);
                     const uint32_t t_sfk = tmem + ((g & 1u) ? kColSfK1 : kColSfK0);
@@ -724,6 +676,11 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 tmem_cp_sf(t_sfv + 4, d1);
             }
             const uint64_t dsfp0 = make_smem_desc(smem_base + SmemLayout::sfp, 0, 128, kSwizzleNone);
+            // MN-major B: 8-key groups 1024 B apart; the second 128-byte-wide atom (columns 128..) is the tile of ones. Moving the start address on moves the
+            // distance to the ones back
+            const uint64_t dv0 = make_smem_desc(v_smem, ones_smem - v_smem, 1024, kSwizzle128B);
+            constexpr uint64_t kDvKeys = (4096u >> 4) - (static_cast<uint64_t>(4096u >> 4) << 16), kDvStage = (kTileBytes >> 4) - (static_cast<uint64_t>(kTileBytes >> 4) << 16);
+            uint64_t dv_st = dv0;
             uint32_t g = 0, n = 0, ph = 0;
             int st = 0;
             bool ok = true;
@@ -743,9 +700,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     if (elect_one_sync()) {
 #pragma unroll
                         for (int kb = 0; kb < 4; ++kb) {
-                            // MN-major B: 8-key groups 1024 B apart; the second 128-byte-wide atom (columns 128..) is the tile of ones
-                            const uint32_t v_addr = v_smem + st * kTileBytes + kb * 4096;
-                            const uint64_t dv = make_smem_desc(v_addr, ones_smem - v_addr, 1024, kSwizzle128B);
+                            const uint64_t dv = dv_st + static_cast<uint64_t>(kb) * kDvKeys;
                             if (kScaled) {
                                 if (kLazy && kb == 0) tmem_cp_sf(t_sfp, dsfp0 + static_cast<uint64_t>(((g & 1u) * kSfBytes) >> 4));
                                 if (kVbs && kb == 0) tmem_cp_sf(t_sfv, make_smem_desc(smem_base + SmemLayout::sfv + st * kSfBytes, 0, 128, kSwizzleNone));
@@ -763,7 +718,8 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         stamp(mma_trace, 3, static_cast<int>(g), 4);
                     }
                     ++g;
-                    if (++st == kStages) { st = 0; ph ^= 1u; }
+                    dv_st += kDvStage;
+                    if (++st == kStages) { st = 0; ph ^= 1u; dv_st = dv0; }
                 }
             }
         }
@@ -806,10 +762,9 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // free
         bool p_ready = false;
         auto hand_over_p = [&]() {
-            if (!p_ready) return;
             tmem_wait_st();
             tc_fence_before_sync();
-            mbar_arrive(bar_p_full(par));
+            mbar_arrive_if(bar_p_full(par), p_ready);
             p_ready = false;
         };
         const bool want_fin = kSplit || p.lse_nat != nullptr || cta_traced || kCluster != kNoCluster;   // does anything read the final reference?
@@ -949,7 +904,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     }
                     if (c == 24) {
                         st_shared_v2(ref_slot(g), __float_as_uint(ref), g);
-                        pv_seen = k == 0 || mbar_test_wait(bar_o_done(par), (k - 1u) & 1u);   // probed ahead: P V of this parity's previous tile
+                        pv_seen = mbar_test_wait(bar_o_done(par), (k - 1u) & 1u);   // probed ahead: P V of this parity's previous tile (true for the first: the phase before a new barrier's)
                     }
                     if (c == 32 && j > 0) prev = ld_shared_v2(ref_slot(g - 1u));
                     if (c >= kConvDepth) conv_finish(c - kConvDepth);

@@ -24,6 +24,9 @@ __device__ __forceinline__ void fence_mbar_init() {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_if(uint32_t bar, bool live) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(static_cast<uint32_t>(live)) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -75,7 +78,7 @@ constexpr long long kWaitBudgetCycles = 400000000LL;
 // already flagged a failure (`*abort_flag != 0`, a shared-memory word). A failed try_wait has already been parked by the hardware
 // for a time slice, so the flag and the clock are only looked at on every eighth failure.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, long long budget = kWaitBudgetCycles) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
     const long long t0 = clock64();
     for (uint32_t spins = 1;; ++spins) {
         if (mbar_try_wait(bar, parity)) return true;
@@ -170,6 +173,15 @@ __device__ __forceinline__ bool elect_one_sync() {
         : "=r"(pred));
     return pred != 0;
 }
+
+// ----------------------------------------------------------------------------------------------- 4-byte asynchronous copies
+// global -> shared (generic proxy); with `bytes` 0 nothing is read and the word becomes 0
+__device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src, uint32_t bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// one arrival on `bar` (already in its count) when this thread's copies so far have landed
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // ----------------------------------------------------------------------------------------------- fences
 __device__ __forceinline__ void fence_proxy_async_smem() {
