@@ -386,48 +386,77 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // ---- one-time setup ----
     if (threadIdx.x == 0) stamp(cta_traced ? p.trace : nullptr, 2, 30, 0);   // kernel entry
-    if (threadIdx.x == 0) {
-        *abort_flag = 0u;
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(bar_q_full(b), 1 + 32);   // the TMA's expect-tx arrive + the producer lanes' scale copies
-            mbar_init(bar_q_empty(b), 1);
-            mbar_init(bar_s_full(b), 1);
-            mbar_init(bar_s_free(b), kRows);
-            mbar_init(bar_p_full(b), kRows);
-            mbar_init(bar_o_done(b), 1);
+    // The producers' copies of scale bytes: E8M0 words of 128 rows -> [row % 32][row / 32][4], the layout tcgen05.cp 32x128b.warpx4 spreads over the four lane
+    // quadrants. Lane l copies rows l, l + 32, ...; the copies arrive on the tile's barrier when they have landed (32 arrivals).
+    auto copy_q_scales = [&](const Item& it, uint32_t qb) {
+        const uint32_t dst = sfq_smem + qb * kSfBytes + static_cast<uint32_t>(lane) * 16u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t lr = lane + 32 * i;
+            const uint32_t r = min(it.row0 + (lr >> pack_shift), p.S - 1u);   // rows past the sequence reuse the last row's scales (block3.rs:110-113)
+            const uint32_t head = it.head + (lr & ((1u << pack_shift) - 1u));
+            cp_async_4(dst + 4u * i, p.q_descale + static_cast<size_t>(it.batch) * p.qs_batch_stride + (static_cast<size_t>(r) * p.H + head) * 4u, 4u);
         }
-        for (int st = 0; st < kStages; ++st) {
-            mbar_init(bar_k_full(st), 1 + 32);
-            mbar_init(bar_k_empty(st), 1);
-            mbar_init(bar_v_full(st), kVbs ? 2 : 1);   // with V block scales: the TMA's expect-tx arrive + the arrive that follows the scale bytes
-            mbar_init(bar_v_empty(st), 1);
-        }
-        mbar_init(bar_o_free, kRows);   // the epilogue warpgroup's 128 threads
-        mbar_init(bar_o_full, 1);
-        mbar_init(bar_peer_rdy, kCut ? 1u << p.cut_log2 : 1u);
-        mbar_init(bar_peer_data, kRows);
+        cp_async_arrive(bar_q_full(qb));
+    };
+    // `src`: the scale word of this lane's first key of the tile; `keys_left`: sequence keys from there on (keys past the sequence: zeros; their data is zero-filled too)
+    auto copy_k_scales = [&](const uint8_t* src, int keys_left, int st) {
+        const uint32_t dst = sfk_smem + static_cast<uint32_t>(st) * kSfBytes + static_cast<uint32_t>(lane) * 16u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cp_async_4(dst + 4u * i, src + static_cast<size_t>(i) * (32u * p.HK * 4u), 32 * i < keys_left ? 4u : 0u);
+        cp_async_arrive(bar_k_full(st));
+    };
+    auto k_scales_of = [&](const Item& it) { return p.k_descale + static_cast<size_t>(it.batch) * p.ks_batch_stride + (static_cast<size_t>(it.key_lo + lane) * p.HK + it.kv_head) * 4u; };
+    if (warp == kKProducerWarp) {
+        // This warp sets the barriers up and sends out the CTA's first copies (Q, K and V tile of its first item, their scales) while the others are still at
+        // the rest of the set-up: what a launch starts with is the wait for them. From the role's own loop they went out 600 clocks later (launches in a graph:
+        // B1 H2 S256 5.83 us, so 5.42; one row block of 16 tiles 13.30 and 12.86).
+        if (lane < 3) prefetch_tmap(lane == 0 ? &tm_q : lane == 1 ? &tm_k : &tm_v);
+        const uint32_t l = static_cast<uint32_t>(lane);
+        uint32_t count = 1u;                                   // of barrier l (SmemLayout::bars); lanes 30 and 31: peer_rdy and peer_data
+        if (l < 2u || (l >= 4u && l < 8u)) count = 1u + 32u;     // q_full, k_full: the TMA's expect-tx arrive + the producer lanes' scale copies
+        if (kVbs && l >= 12u && l < 16u) count = 2u;             // v_full: the same + the arrive that follows V's scale bytes
+        if (l >= 22u && l < 26u) count = kRows;                  // s_free, p_full
+        if (l == 28u || l == 31u) count = kRows;                 // o_free (the epilogue warpgroup's 128 threads), peer_data
+        if (l == 30u) count = kCut ? 1u << p.cut_log2 : 1u;
+        static_assert(kStages == 4, "the barriers' order");
+        mbar_init(bar0 + 8u * (l < 30u ? l : l + 4u), count);
+        if (lane == 0) *abort_flag = 0u;
         fence_mbar_init();
+        __syncwarp();
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // (see below)
+        if (blockIdx.x < n_items) {
+            const Item it = decode_item<kSplit, kCausal, kCluster, kPack>(blockIdx.x, p);
+            if (elect_one_sync()) {
+                mbar_arrive_expect_tx(bar_q_full(0), kTileBytes);
+                tma_load_4d(q_smem, &tm_q, bar_q_full(0), 0, static_cast<int>(it.head), static_cast<int>(it.row0), static_cast<int>(it.batch));
+                stamp(cta_traced ? p.trace : nullptr, 2, 0, 6);
+                mbar_arrive_expect_tx(bar_k_full(0), kTileBytes);
+                tma_load_4d(k_smem, &tm_k, bar_k_full(0), 0, static_cast<int>(it.kv_head), static_cast<int>(it.key_lo), static_cast<int>(it.batch));
+                mbar_arrive_expect_tx(bar_v_full(0), kTileBytes);
+                tma_load_4d(v_smem, &tm_v, bar_v_full(0), 0, static_cast<int>(it.kv_head), static_cast<int>(it.key_lo), static_cast<int>(it.batch));
+            }
+            __syncwarp();
+            copy_q_scales(it, 0u);
+            copy_k_scales(k_scales_of(it), static_cast<int>(p.SK - it.key_lo) - lane, 0);
+        }
     }
-    if ((kLazy || kVbs) && threadIdx.x >= 256 && threadIdx.x < 384) {
-        reinterpret_cast<uint32_t*>(smem_gen + SmemLayout::sf_one)[threadIdx.x - 256] = 0x7F7F7F7Fu;
+    if ((kLazy || kVbs) && threadIdx.x >= 128 && threadIdx.x < 256) {
+        reinterpret_cast<uint32_t*>(smem_gen + SmemLayout::sf_one)[threadIdx.x - 128] = 0x7F7F7F7Fu;
         fence_proxy_async_smem();
     }
-    if (threadIdx.x < 256) {
-        for (int i = 0; i < 4; ++i) reinterpret_cast<uint32_t*>(smem_gen + SmemLayout::ones)[threadIdx.x + 256 * i] = 0x38383838u;
+    if (threadIdx.x >= 256) {
+        const uint32_t t = threadIdx.x - 256u;
+        for (int i = 0; i < 4; ++i) reinterpret_cast<uint32_t*>(smem_gen + SmemLayout::ones)[t + 256 * i] = 0x38383838u;
         // the 1024 reference hand-over slots start with a tile counter no tile has
-        for (int i = 0; i < 4; ++i) reinterpret_cast<uint2*>(smem_gen + SmemLayout::xref)[threadIdx.x + 256 * i] = make_uint2(0u, 0xFFFFFFFFu);
-        reinterpret_cast<uint32_t*>(smem_gen + SmemLayout::sfp)[threadIdx.x] = 0x7F7F7F7Fu;
+        for (int i = 0; i < 4; ++i) reinterpret_cast<uint2*>(smem_gen + SmemLayout::xref)[t + 256 * i] = make_uint2(0u, 0xFFFFFFFFu);
+        reinterpret_cast<uint32_t*>(smem_gen + SmemLayout::sfp)[t] = 0x7F7F7F7Fu;
         fence_proxy_async_smem();
     }
     if (warp == kMmaWarp) {
         tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
         tmem_relinquish();
     }
-    if (warp == kKProducerWarp && lane == 0) {
-        prefetch_tmap(&tm_q);
-        prefetch_tmap(&tm_k);
-    }
-    if (warp == kVProducerWarp && lane == 0) prefetch_tmap(&tm_v);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -444,8 +473,8 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             cluster_joined = true;
         }
     };
-    // nothing above touches global memory; everything below may read what the previous grid in the stream wrote (a quantiser that is still writing the
-    // scales as this grid starts, for one): by TMA or with volatile loads, never through __ldg, which the compiler may move in front of the wait
+    // nothing above but the first copies, which wait for themselves, touches global memory; everything below may read what the previous grid in the stream wrote
+    // (a quantiser that is still writing the scales as this grid starts, for one): by TMA or with volatile loads, never through __ldg, which the compiler may move in front of the wait
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x == 0) stamp(cta_traced ? p.trace : nullptr, 2, 30, 2);   // setup done
 
@@ -465,35 +494,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // the loads of the first five (B1 H37 S512 Skv2048, 148 items of 16 tiles: 16.3 us, so 15.2; B4 H8 S2048 48.7, so 47.7).
         auto producer = [&](auto is_k_c) {
             constexpr bool kIsK = decltype(is_k_c)::value;
-            // E8M0 words of 128 rows -> [row % 32][row / 32][4] (the layout tcgen05.cp 32x128b.warpx4 spreads over the four lane quadrants): lane l copies
-            // rows l, l + 32, ... The copies arrive on the tile's barrier when they have landed (32 arrivals).
-            auto copy_q_scales = [&](const Item& it, uint32_t qb) {
-                const uint32_t dst = sfq_smem + qb * kSfBytes + static_cast<uint32_t>(lane) * 16u;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint32_t lr = lane + 32 * i;
-                    const uint32_t r = min(it.row0 + (lr >> pack_shift), p.S - 1u);   // rows past the sequence reuse the last row's scales (block3.rs:110-113)
-                    const uint32_t head = it.head + (lr & ((1u << pack_shift) - 1u));
-                    cp_async_4(dst + 4u * i, p.q_descale + static_cast<size_t>(it.batch) * p.qs_batch_stride + (static_cast<size_t>(r) * p.H + head) * 4u, 4u);
-                }
-                cp_async_arrive(bar_q_full(qb));
-            };
-            const uint32_t row_step = 32u * p.HK * 4u, tile_step = 4u * row_step;   // of the K scales: bytes between a lane's four keys / between key tiles
-            // The CTA's first copies (Q tile and first K tile, first V tile of its first item) go out before anything else of the role's set-up.
-            if (blockIdx.x < n_items && elect_one_sync()) {
-                const Item it = decode_item<kSplit, kCausal, kCluster, kPack>(blockIdx.x, p);
-                if (kIsK) {
-                    mbar_arrive_expect_tx(bar_q_full(0), kTileBytes);
-                    tma_load_4d(q_smem, &tm_q, bar_q_full(0), 0, static_cast<int>(it.head), static_cast<int>(it.row0), static_cast<int>(it.batch));
-                    stamp(cta_traced ? p.trace : nullptr, 2, 0, 6);
-                    mbar_arrive_expect_tx(bar_k_full(0), kTileBytes);
-                    tma_load_4d(k_smem, &tm_k, bar_k_full(0), 0, static_cast<int>(it.kv_head), static_cast<int>(it.key_lo), static_cast<int>(it.batch));
-                } else {
-                    stamp(cta_traced ? p.trace : nullptr, 3, 0, 6);
-                    mbar_arrive_expect_tx(bar_v_full(0), kTileBytes);
-                    tma_load_4d(v_smem, &tm_v, bar_v_full(0), 0, static_cast<int>(it.kv_head), static_cast<int>(it.key_lo), static_cast<int>(it.batch));
-                }
-            }
+            const uint32_t tile_step = 128u * p.HK * 4u;   // of the K scales: bytes between key tiles
             uint32_t g = 0, n = 0, ph = 0, q_issued = 0;   // g: the running tile counter
             int st = 0;
             bool ok = true;
@@ -508,11 +509,10 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         mbar_arrive_expect_tx(bar_q_full(qb), kTileBytes);
                         tma_load_4d(q_smem + qb * kTileBytes, &tm_q, bar_q_full(qb), 0, static_cast<int>(it.head), static_cast<int>(it.row0), static_cast<int>(it.batch));
                     }
-                    copy_q_scales(it, qb);
+                    if (n > 0) copy_q_scales(it, qb);
                     ++q_issued;
                 }
-                // scale word of this lane's first key of the tile; sequence keys from the tile's first key on (lanes compare against it)
-                const uint8_t* k_scales = p.k_descale + static_cast<size_t>(it.batch) * p.ks_batch_stride + (static_cast<size_t>(it.key_lo + lane) * p.HK + it.kv_head) * 4u;
+                const uint8_t* k_scales = k_scales_of(it);
                 int keys_left = static_cast<int>(p.SK - it.key_lo) - lane;
                 float* k_trace = cta_traced ? p.trace : nullptr;   // stamps are indexed by the running tile counter
                 int key = static_cast<int>(it.key_lo);
@@ -534,10 +534,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             mbar_arrive_expect_tx(bar_k_full(st), kTileBytes);
                             tma_load_4d(k_smem + st * kTileBytes, &tm_k, bar_k_full(st), 0, static_cast<int>(it.kv_head), key, static_cast<int>(it.batch));
                         }
-                        const uint32_t dst = sfk_smem + static_cast<uint32_t>(st) * kSfBytes + static_cast<uint32_t>(lane) * 16u;
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) cp_async_4(dst + 4u * i, k_scales + i * row_step, 32 * i < keys_left ? 4u : 0u);   // (keys past the sequence: zeros; their data is zero-filled too)
-                        cp_async_arrive(bar_k_full(st));
+                        if (g > 0) copy_k_scales(k_scales, keys_left, st);   // (the CTA's first tile, and the first item's Q, went out in the set-up)
                         k_scales += tile_step;
                         keys_left -= kKeys;
                     }
