@@ -27,9 +27,13 @@ __device__ __forceinline__ uint32_t e4m3x2(float lo, float hi) {
 
 // Programmatic dependent launch, both sides: the launch behind this one may be scheduled while this grid runs, and nothing above the wait touches
 // global memory. A short prompt's chain (Q, K, V, attention) is launches more than work.
-__device__ __forceinline__ void pdl_begin() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Asks L2 for the line at `p`, one thread per 128 bytes of a warp's 16-byte vectors. Allowed in front of the wait: nothing is read, and L2 is where a write of the grid
+// before would land too. The first vectors of a grid then come from DRAM while the last blocks of the grid before still run.
+__device__ __forceinline__ void prefetch_vec(const uint4* p) {
+    if ((threadIdx.x & 7u) == 0u) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
 // A 16-byte read-once load. Volatile, so that it stays behind the wait above, and not of the non-coherent kind, which is for data that nothing writes while
@@ -80,11 +84,17 @@ __device__ __forceinline__ void quantize_qk_vec(const uint4 raw, bool live, floa
 template <int kVecs>
 __global__ void __launch_bounds__(256) quantize_qk_kernel(const uint4* __restrict__ x, unsigned long long rows, float mul,
                                                           uint2* __restrict__ out, uint32_t* __restrict__ scales) {
-    pdl_begin();
+    pdl_launch();
     const unsigned long long n_threads = rows * 16ull, step = static_cast<unsigned long long>(gridDim.x) * (256u * kVecs);
     const unsigned lane = threadIdx.x & 31u;
-    // t0: the warp's first vector; whole warps stay in the loop together: the shuffles need all lanes
-    for (unsigned long long t0 = static_cast<unsigned long long>(blockIdx.x) * (256u * kVecs) + (threadIdx.x & ~31u); t0 < n_threads; t0 += step) {
+    // the warp's first vector; whole warps stay in the loop together: the shuffles need all lanes
+    const unsigned long long first = static_cast<unsigned long long>(blockIdx.x) * (256u * kVecs) + (threadIdx.x & ~31u);
+#pragma unroll
+    for (int i = 0; i < kVecs; ++i) {
+        if (first + lane + 256u * i < n_threads) prefetch_vec(x + first + lane + 256u * i);
+    }
+    pdl_wait();
+    for (unsigned long long t0 = first; t0 < n_threads; t0 += step) {
         uint4 raw[kVecs];
 #pragma unroll
         for (int i = 0; i < kVecs; ++i) {
@@ -136,12 +146,24 @@ __device__ __forceinline__ uint2 quantize_v_vec(const uint4 raw, float vd, float
     return make_uint2(b[0], b[1]);
 }
 
+// descale = {0, 0} in front of the running maximum. A kernel of the chain and not a memset: around a memset the grids before and behind it start and end alone.
+__global__ void clear_descale_kernel(float* descale) {
+    pdl_launch();
+    pdl_wait();
+    if (threadIdx.x < 2u) descale[threadIdx.x] = 0.0f;
+}
+
 template <int kVecs>
 __global__ void __launch_bounds__(256) amax_kernel(const uint4* __restrict__ x, unsigned long long n_vec, uint32_t* __restrict__ amax_bits) {
     float amax = 0.0f;
-    const unsigned long long step = static_cast<unsigned long long>(gridDim.x) * (256u * kVecs);
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    for (unsigned long long t0 = static_cast<unsigned long long>(blockIdx.x) * (256u * kVecs) + threadIdx.x; t0 < n_vec; t0 += step) {
+    const unsigned long long step = static_cast<unsigned long long>(gridDim.x) * (256u * kVecs), first = static_cast<unsigned long long>(blockIdx.x) * (256u * kVecs) + threadIdx.x;
+    pdl_launch();
+#pragma unroll
+    for (int i = 0; i < kVecs; ++i) {
+        if (first + 256u * i < n_vec) prefetch_vec(x + first + 256u * i);
+    }
+    pdl_wait();
+    for (unsigned long long t0 = first; t0 < n_vec; t0 += step) {
         uint4 raw[kVecs];
 #pragma unroll
         for (int i = 0; i < kVecs; ++i) raw[i] = t0 + 256u * i < n_vec ? ld_vec(x + t0 + 256u * i) : make_uint4(0u, 0u, 0u, 0u);
@@ -163,7 +185,8 @@ __global__ void __launch_bounds__(256) amax_kernel(const uint4* __restrict__ x, 
 template <int kVecs>
 __global__ void __launch_bounds__(256) quantize_v_kernel(const uint4* __restrict__ x, unsigned long long n_vec, uint2* __restrict__ out,
                                                          float* __restrict__ descale) {
-    pdl_begin();
+    pdl_launch();
+    pdl_wait();
     const float amax = __uint_as_float(reinterpret_cast<const volatile uint32_t*>(descale)[1]);
     const float vd = v_descale_of(amax);
     if (blockIdx.x == 0 && threadIdx.x == 0) descale[0] = vd;
@@ -194,12 +217,18 @@ quantize_v_small_kernel(const uint4* __restrict__ x, unsigned n_vec, uint2* __re
     // A CTA's shared memory may only be written by another one once it is known to have started: every thread arrives here and waits in front of the
     // exchange, behind the loads. (Being scheduled as one cluster does not give that order, nor does the wait for the grid before.)
     asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
-    pdl_begin();
+    pdl_launch();
     __shared__ float part[kSmallThreads / 32];
     __shared__ float cta_amax[kSmallCtas];   // [source CTA], written by all of them
     const cg::cluster_group cluster = cg::this_cluster();
     const unsigned tid = blockIdx.x * kSmallThreads + threadIdx.x;
     uint4 raw[kSmallVecs];
+#pragma unroll
+    for (unsigned i = 0; i < kSmallVecs; ++i) {
+        const unsigned t = tid + i * (kSmallCtas * kSmallThreads);
+        if (t < n_vec) prefetch_vec(x + t);
+    }
+    pdl_wait();
 #pragma unroll
     for (unsigned i = 0; i < kSmallVecs; ++i) {
         const unsigned t = tid + i * (kSmallCtas * kSmallThreads);
@@ -273,13 +302,11 @@ cudaError_t launch_quantize_v(const void* x_bf16, unsigned long long n_elems, vo
     const uint4* x = static_cast<const uint4*>(x_bf16);
     uint2* out = static_cast<uint2*>(out_e4m3);
     if (n_vec <= kSmallMax) return launch_pdl(quantize_v_small_kernel, kSmallCtas, kSmallThreads, stream, x, static_cast<unsigned>(n_vec), out, descale);
-    cudaError_t e = cudaMemsetAsync(descale, 0, 8, stream);   // [0] the descale, [1] the running maximum's bits
+    cudaError_t e = launch_pdl(clear_descale_kernel, 1u, 32u, stream, descale);   // [0] the descale, [1] the running maximum's bits
     if (e != cudaSuccess) return e;
     const bool wide = n_vec >= kWideVecs;
     const unsigned grid = grid_for(n_vec, wide ? 4u : 1u);
-    if (wide) amax_kernel<4><<<grid, 256, 0, stream>>>(x, n_vec, reinterpret_cast<uint32_t*>(descale) + 1);
-    else amax_kernel<1><<<grid, 256, 0, stream>>>(x, n_vec, reinterpret_cast<uint32_t*>(descale) + 1);
-    e = cudaGetLastError();
+    e = launch_pdl(wide ? amax_kernel<4> : amax_kernel<1>, grid, 256u, stream, x, n_vec, reinterpret_cast<uint32_t*>(descale) + 1);
     if (e != cudaSuccess) return e;
     return launch_pdl(wide ? quantize_v_kernel<4> : quantize_v_kernel<1>, grid, 256u, stream, x, n_vec, out, descale);
 }
