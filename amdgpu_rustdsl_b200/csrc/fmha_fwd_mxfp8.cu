@@ -433,6 +433,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 stamp(cta_traced ? p.trace : nullptr, 2, 0, 6);
                 mbar_arrive_expect_tx(bar_k_full(0), kTileBytes);
                 tma_load_4d(k_smem, &tm_k, bar_k_full(0), 0, static_cast<int>(it.kv_head), static_cast<int>(it.key_lo), static_cast<int>(it.batch));
+                stamp(cta_traced ? p.trace : nullptr, 3, 0, 6);
                 mbar_arrive_expect_tx(bar_v_full(0), kTileBytes);
                 tma_load_4d(v_smem, &tm_v, bar_v_full(0), 0, static_cast<int>(it.kv_head), static_cast<int>(it.key_lo), static_cast<int>(it.batch));
             }
