@@ -407,6 +407,15 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         cp_async_arrive(bar_k_full(st));
     };
     auto k_scales_of = [&](const Item& it) { return p.k_descale + static_cast<size_t>(it.batch) * p.ks_batch_stride + (static_cast<size_t>(it.key_lo + lane) * p.HK + it.kv_head) * 4u; };
+    // Launched as clusters (items are cut between their CTAs): the partner's barriers must exist before anything can arrive on them. Every thread arrives on
+    // the cluster's barrier in the set-up, the warp that sets the barriers up behind that, all in front of the wait for the grid before, and waits for it only where it
+    // first touches the partner (the epilogue warpgroup, the score MMA warp) or, failing that, at the end; by then the partner has long arrived. Behind
+    // that wait the arrivals stand in every launch's way (back to back: B1 H8 HK2 S512 Skv4096 cut in 8 16.4 us, so 15.9; B1 H10 S2048 Skv8192 as pairs 67.5 and 67.2).
+    constexpr bool paired = kCluster != kNoCluster;
+    auto arrive_cluster = [&]() {
+        if (paired) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    };
+    if (warp != kKProducerWarp) arrive_cluster();
     if (warp == kKProducerWarp) {
         // This warp sets the barriers up and sends out the CTA's first copies (Q, K and V tile of its first item, their scales) while the others are still at
         // the rest of the set-up: what a launch starts with is the wait for them. From the role's own loop they went out 600 clocks later (launches in a graph:
@@ -424,6 +433,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         if (lane == 0) *abort_flag = 0u;
         fence_mbar_init();
         __syncwarp();
+        arrive_cluster();
         asm volatile("griddepcontrol.wait;" ::: "memory");   // (see below)
         if (blockIdx.x < n_items) {
             const Item it = decode_item<kSplit, kCausal, kCluster, kPack>(blockIdx.x, p);
@@ -462,12 +472,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    // launched as clusters (items are cut between their CTAs): the partner's barriers must exist before anything can arrive on them
-    // Every thread arrives on the cluster's barrier here and waits for it only where it first touches the partner (the epilogue
-    // warpgroup, the score MMA warp) or, failing that, at the end; by then the partner has long arrived, so nobody stands still for it.
-    constexpr bool paired = kCluster != kNoCluster;
     bool cluster_joined = !paired;
-    if (paired) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     auto join_cluster = [&]() {
         if (!cluster_joined) {
             asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
