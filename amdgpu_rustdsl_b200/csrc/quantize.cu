@@ -25,13 +25,15 @@ __device__ __forceinline__ uint32_t e4m3x2(float lo, float hi) {
     return h;
 }
 
-// Programmatic dependent launch, both sides: the launch behind this one may be scheduled while this grid runs, and nothing above the wait touches
-// global memory. A short prompt's chain (Q, K, V, attention) is launches more than work.
+// Programmatic dependent launch, both sides: the launch behind this one may be scheduled while this grid runs, and above the wait nothing reads or writes
+// global memory: there are only the hints below. A short prompt's chain (Q, K, V, attention) is launches more than work.
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Asks L2 for the line at `p`, one thread per 128 bytes of a warp's 16-byte vectors. Allowed in front of the wait: nothing is read, and L2 is where a write of the grid
-// before would land too. The first vectors of a grid then come from DRAM while the last blocks of the grid before still run.
+// Asks L2 for the line at `p`, one thread per 128 bytes of a warp's 16-byte vectors (all lines of them where x is 128-byte aligned, all but the last elsewhere). Allowed
+// in front of the wait: nothing is read, and L2 is where a write of the grid before would land too. Of the forms with one vector per thread, whose grids are a few us long:
+// launches in a graph, Q, K and V of B1 H8 HK2 S1000 6.6 us without and 6.0 with it, B1 H16 HK4 S2048 11.1 and 10.5. The wide forms ask for nothing: their first
+// 19 MB, asked for while the grid before still streams, cost more than they save (B8 H32 HK8 S4096 118.4 us without and 122.7 with it).
 __device__ __forceinline__ void prefetch_vec(const uint4* p) {
     if ((threadIdx.x & 7u) == 0u) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
@@ -89,10 +91,7 @@ __global__ void __launch_bounds__(256) quantize_qk_kernel(const uint4* __restric
     const unsigned lane = threadIdx.x & 31u;
     // the warp's first vector; whole warps stay in the loop together: the shuffles need all lanes
     const unsigned long long first = static_cast<unsigned long long>(blockIdx.x) * (256u * kVecs) + (threadIdx.x & ~31u);
-#pragma unroll
-    for (int i = 0; i < kVecs; ++i) {
-        if (first + lane + 256u * i < n_threads) prefetch_vec(x + first + lane + 256u * i);
-    }
+    if (kVecs == 1 && first + lane < n_threads) prefetch_vec(x + first + lane);
     pdl_wait();
     for (unsigned long long t0 = first; t0 < n_threads; t0 += step) {
         uint4 raw[kVecs];
@@ -158,10 +157,7 @@ __global__ void __launch_bounds__(256) amax_kernel(const uint4* __restrict__ x, 
     float amax = 0.0f;
     const unsigned long long step = static_cast<unsigned long long>(gridDim.x) * (256u * kVecs), first = static_cast<unsigned long long>(blockIdx.x) * (256u * kVecs) + threadIdx.x;
     pdl_launch();
-#pragma unroll
-    for (int i = 0; i < kVecs; ++i) {
-        if (first + 256u * i < n_vec) prefetch_vec(x + first + 256u * i);
-    }
+    if (kVecs == 1 && first < n_vec) prefetch_vec(x + first);
     pdl_wait();
     for (unsigned long long t0 = first; t0 < n_vec; t0 += step) {
         uint4 raw[kVecs];
