@@ -13,6 +13,7 @@
 namespace {
 
 using b200mx::AttnParams;
+using b200mx::current_sm_count;
 
 static_assert(sizeof(fmha_mxfp8_attn_args) == 656, "vs128/t128 kernarg size");
 static_assert(sizeof(fmha_mxfp8_kvsplit_args) == 648, "kvsplit kernarg size");
@@ -213,22 +214,6 @@ uint32_t log2_u32(uint32_t x) {
     return l;
 }
 
-// SMs of the current device (asked once per device), or a B200's where there is none
-int current_sm_count() {
-    static std::atomic<int> known[64];
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
-        n = known[dev].load(std::memory_order_relaxed);
-        if (n > 0) return n;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0) {
-            known[dev].store(n, std::memory_order_relaxed);
-            return n;
-        }
-    }
-    (void)cudaGetLastError();
-    return 148;
-}
-
 std::atomic<float*> g_trace{nullptr};
 
 int launch_attention_kernel(int kernel, const void* args, const uint32_t grid[3], cudaStream_t stream) {
@@ -351,6 +336,20 @@ int launch_attention_kernel(int kernel, const void* args, const uint32_t grid[3]
 }  // namespace
 
 namespace b200mx {
+int current_sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+        n = known[dev].load(std::memory_order_relaxed);
+        if (n > 0) return n;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0) {
+            known[dev].store(n, std::memory_order_relaxed);
+            return n;
+        }
+    }
+    (void)cudaGetLastError();
+    return 148;
+}
 int encode_partial_map(CUtensorMap* m, void* base, uint64_t seq, uint64_t heads, uint64_t batches, uint64_t splits, bool f32) {
     return make_partial_map(m, base, seq, heads, batches, splits, f32);
 }

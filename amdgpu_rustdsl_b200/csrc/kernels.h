@@ -102,6 +102,7 @@ cudaError_t launch_mma_issue_ceiling(int iters, int ctas, uint32_t* status, cuda
 // wait_selftest.cu: one CTA lets a bounded wait run out (budget in SM cycles) and reports what happened in *word; *ms = kernel time.
 cudaError_t run_bounded_wait_selftest(long long budget_cycles, cudaStream_t stream, uint32_t* word, float* ms);
 
+int current_sm_count();   // SMs of the current device (asked once per device), or a B200's where there is none
 uint32_t* device_status_word();   // address of the per-device status word (device pointer)
 
 }  // namespace b200mx

@@ -191,15 +191,15 @@ def _raw_stream(torch, dev):
     return get(dev.index or 0) if get is not None else torch.cuda.current_stream(dev).cuda_stream
 
 
-def _on_device(torch, dev, stream, launch):
-    """``launch(stream handle)`` with the tensors' device current: the library works on the current device (status word, SM count, kernel attributes, stream 0).
+def _on_device(torch, dev, stream, launch, *args):
+    """``launch(*args, stream handle)`` with the tensors' device current: the library works on the current device (status word, SM count, kernel attributes, stream 0).
     Entering and leaving it, and building the stream object, cost a few us a call, which is what a short prompt's chain of calls then waits for."""
     if stream is None:
         stream = _raw_stream(torch, dev)
     if torch.cuda.current_device() == (dev.index or 0):
-        return launch(stream)
+        return launch(*args, C.c_void_p(stream))
     with torch.cuda.device(dev):
-        return launch(stream)
+        return launch(*args, C.c_void_p(stream))
 
 
 def _launch_dispatched(unsplit, lib, q, k, v, q_scale, k_scale, v_scale, out, path, splits, stream, check, flags, v_blockscale, lse, B, S, H, SK, HK, record):
@@ -269,12 +269,13 @@ def quantize_qk(x, out, out_scales, *, mul=1.0, stream=None):
     (tests/gpu/ref_host.cpp:239-254) on the device; pass ``mul=Q_PRESCALE`` for Q and 1 for K."""
     import torch
     lib = _abi.load()
-    rows = x.numel() // D
+    n = x.numel()
+    rows = n // D
     if x.dtype != torch.bfloat16 or x.shape[-1] != D or not x.is_contiguous() or not x.is_cuda:
         raise ValueError("quantize_qk: x must be a contiguous CUDA bf16 tensor [..., 128]")
-    if out.numel() != x.numel() or out.element_size() != 1 or not out.is_contiguous() or _nbytes(out_scales) < rows * 4:
+    if out.numel() != n or out.element_size() != 1 or not out.is_contiguous() or _nbytes(out_scales) < rows * 4:
         raise ValueError("quantize_qk: out must hold one byte per element and out_scales 4 bytes per row")
-    rc = _on_device(torch, x.device, stream, lambda raw: lib.fmha_mxfp8_quantize_qk(x.data_ptr(), rows, float(mul), out.data_ptr(), out_scales.data_ptr(), C.c_void_p(raw)))
+    rc = _on_device(torch, x.device, stream, lib.fmha_mxfp8_quantize_qk, x.data_ptr(), rows, float(mul), out.data_ptr(), out_scales.data_ptr())
     if rc:
         raise RuntimeError(f"fmha_mxfp8_quantize_qk failed with code {rc}")
 
@@ -283,10 +284,11 @@ def quantize_v(x, out, v_descale, *, stream=None):
     """bf16 ``x`` -> e4m3 bytes ``out`` with one f32 descale written to ``v_descale[0]`` (f32 buffer, the contract asks for >= 4096 bytes)."""
     import torch
     lib = _abi.load()
-    if x.dtype != torch.bfloat16 or not x.is_contiguous() or not x.is_cuda or x.numel() % 8:
+    n = x.numel()
+    if x.dtype != torch.bfloat16 or not x.is_contiguous() or not x.is_cuda or n % 8:
         raise ValueError("quantize_v: x must be a contiguous CUDA bf16 tensor with a multiple of 8 elements")
-    if out.numel() != x.numel() or out.element_size() != 1 or not out.is_contiguous() or _nbytes(v_descale) < 8:
+    if out.numel() != n or out.element_size() != 1 or not out.is_contiguous() or _nbytes(v_descale) < 8:
         raise ValueError("quantize_v: out must hold one byte per element and v_descale at least 8 bytes")
-    rc = _on_device(torch, x.device, stream, lambda raw: lib.fmha_mxfp8_quantize_v(x.data_ptr(), x.numel(), out.data_ptr(), v_descale.data_ptr(), C.c_void_p(raw)))
+    rc = _on_device(torch, x.device, stream, lib.fmha_mxfp8_quantize_v, x.data_ptr(), n, out.data_ptr(), v_descale.data_ptr())
     if rc:
         raise RuntimeError(f"fmha_mxfp8_quantize_v failed with code {rc}")
