@@ -31,9 +31,9 @@ __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.laun
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Asks L2 for the line at `p`, one thread per 128 bytes of a warp's 16-byte vectors (all lines of them where x is 128-byte aligned, all but the last elsewhere). Allowed
-// in front of the wait: nothing is read, and L2 is where a write of the grid before would land too. Of the forms with one vector per thread, whose grids are a few us long:
-// launches in a graph, Q, K and V of B1 H8 HK2 S1000 6.6 us without and 6.0 with it, B1 H16 HK4 S2048 11.1 and 10.5. The wide forms ask for nothing: their first
-// 19 MB, asked for while the grid before still streams, cost more than they save (B8 H32 HK8 S4096 118.4 us without and 122.7 with it).
+// in front of the wait: nothing is read, and L2 is where a write of the grid before would land too. A grid's first vectors then come from DRAM while the last blocks of the
+// grid before still run. Launches in a graph, without and with it: Q, K and V of B1 H8 HK2 S1000 6.6 and 6.0 us, B1 H16 HK4 S2048 11.1 and 10.5; Q or K of 1.2 M vectors 6.8
+// and 6.3, of 16.8 M 66.8 and 66.1; V of 2.1 M 17.1 and 16.8, of 16.8 M 113.5 and 111.2.
 __device__ __forceinline__ void prefetch_vec(const uint4* p) {
     if ((threadIdx.x & 7u) == 0u) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
@@ -91,7 +91,14 @@ __global__ void __launch_bounds__(256) quantize_qk_kernel(const uint4* __restric
     const unsigned lane = threadIdx.x & 31u;
     // the warp's first vector; whole warps stay in the loop together: the shuffles need all lanes
     const unsigned long long first = static_cast<unsigned long long>(blockIdx.x) * (256u * kVecs) + (threadIdx.x & ~31u);
-    if (kVecs == 1 && first + lane < n_threads) prefetch_vec(x + first + lane);
+    // Behind a branch in the wide form: without it the kernel compiles to 40 registers, not 46, and is slower for it (Q or K of 16.8 M vectors 76.8 us, so 71.5, both with
+    // a grid of 8 CTAs per SM)
+    if (kVecs == 1 || first < n_threads) {
+#pragma unroll
+        for (int i = 0; i < kVecs; ++i) {
+            if (first + lane + 256u * i < n_threads) prefetch_vec(x + first + lane + 256u * i);
+        }
+    }
     pdl_wait();
     for (unsigned long long t0 = first; t0 < n_threads; t0 += step) {
         uint4 raw[kVecs];
@@ -159,7 +166,10 @@ __global__ void __launch_bounds__(256) amax_kernel(const uint4* __restrict__ x, 
     float amax = 0.0f;
     const unsigned long long step = static_cast<unsigned long long>(gridDim.x) * (256u * kVecs), first = static_cast<unsigned long long>(blockIdx.x) * (256u * kVecs) + threadIdx.x;
     pdl_launch();
-    if (kVecs == 1 && first < n_vec) prefetch_vec(x + first);
+#pragma unroll
+    for (int i = 0; i < kVecs; ++i) {
+        if (first + 256u * i < n_vec) prefetch_vec(x + first + 256u * i);
+    }
     pdl_wait();
     for (unsigned long long t0 = first; t0 < n_vec; t0 += step) {
         uint4 raw[kVecs];
@@ -261,9 +271,9 @@ quantize_v_small_kernel(const uint4* __restrict__ x, unsigned n_vec, uint2* __re
     }
 }
 
-// Blocks of 256 threads with `vecs` vectors each; grid-stride beyond 8 CTAs per SM
-int grid_for(unsigned long long n_vec, unsigned vecs) {
-    const unsigned long long blocks = (n_vec + 256u * vecs - 1) / (256u * vecs), cap = 8ull * static_cast<unsigned long long>(current_sm_count());
+// Blocks of 256 threads with `vecs` vectors each; grid-stride beyond `per_sm` CTAs per SM
+int grid_for(unsigned long long n_vec, unsigned vecs, unsigned per_sm = 8u) {
+    const unsigned long long blocks = (n_vec + 256u * vecs - 1) / (256u * vecs), cap = 1ull * per_sm * static_cast<unsigned long long>(current_sm_count());
     return static_cast<int>(blocks < cap ? (blocks ? blocks : 1) : cap);
 }
 
@@ -289,7 +299,9 @@ constexpr unsigned long long kWideVecs = 4ull * 148ull * 2048ull;
 cudaError_t launch_quantize_qk(const void* x_bf16, unsigned long long rows, float mul, void* out_e4m3, void* out_scales, cudaStream_t stream) {
     const unsigned long long n_vec = rows * 16ull;
     const bool wide = n_vec >= kWideVecs;
-    return launch_pdl(wide ? quantize_qk_kernel<4> : quantize_qk_kernel<1>, grid_for(n_vec, wide ? 4u : 1u), 256u, stream, static_cast<const uint4*>(x_bf16), rows, mul,
+    // An SM holds 5 CTAs of the wide form (46 registers): 10 are two whole rounds of them. With 8, whose second round is three fifths of one, 2.1 M vectors took 10.1 us, so
+    // 9.2 (1.6 M: 7.7 and 8.0; 4.2 M: 18.4 and 17.3; 16.8 M: 72.1 and 66.1)
+    return launch_pdl(wide ? quantize_qk_kernel<4> : quantize_qk_kernel<1>, grid_for(n_vec, wide ? 4u : 1u, wide ? 10u : 8u), 256u, stream, static_cast<const uint4*>(x_bf16), rows, mul,
                       static_cast<uint2*>(out_e4m3), static_cast<uint32_t*>(out_scales));
 }
 

@@ -221,3 +221,20 @@ def test_a_chain_of_dependent_launches_reads_what_the_one_before_wrote(shape, ca
             torch.cuda.synchronize()
             assert all(torch.equal(x.view(torch.int16), y.view(torch.int16)) for x, y in zip(got, want))
     assert device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [75775, 75776, 94719, 94720, 94721, 189441, 284161])   # the wide form from its first size on; one round of its grid's loop on 148 SMs, a row more, two and three
+def test_quantize_qk_rounds_of_the_wide_form(rows):
+    torch = pytest.importorskip("torch")
+    from amdgpu_rustdsl_b200 import quantize_qk
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = (torch.randn(rows, 128, generator=g, device="cuda") * torch.exp2(torch.randint(-12, 12, (rows, 1), generator=g, device="cuda").float())).to(torch.bfloat16)
+    y, s = torch.full((rows + 1, 128), 0xAA, dtype=torch.uint8, device="cuda"), torch.full((rows * 4 + 16,), 0xAA, dtype=torch.uint8, device="cuda")
+    quantize_qk(x, y[:rows], s)
+    f = x.view(rows, 4, 32).float()
+    e = (torch.frexp(f.abs().amax(-1)).exponent - 1 - 8 + 127).clamp(0, 254)
+    assert torch.equal(s[: rows * 4].view(rows, 4).int(), e.int())
+    want = torch.ldexp(f, (127 - e)[..., None]).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8).view(rows, 128)
+    assert torch.equal(y[:rows], want)
+    assert (y[rows] == 0xAA).all() and (s[rows * 4:] == 0xAA).all()   # nothing written past the rows
