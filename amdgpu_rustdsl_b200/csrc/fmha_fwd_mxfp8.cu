@@ -20,7 +20,7 @@
 //              the E8M0 factors copied to TMEM with tcgen05.cp. Two score tiles are always ahead of the softmax.
 //   warp  1    Q / K producer: TMA loads of the Q tile (double buffered across items) and of the K ring, plus the 4-byte-per-row scale
 //              bytes of both, which a TMA box cannot express: 4-byte asynchronous copies straight into the 32x16-byte layout tcgen05.cp
-//              expects, arriving on the tile's barrier.
+//              expects, arriving on the tile's barrier. In the set-up it initialises all barriers and sends out the first Q, K and V tiles.
 //   warp  2    P V issuer: O += P_g V_g with P from TMEM and V (keys x head dim, i.e. MN-major B) from shared memory. The B operand
 //              is 144 wide: 128 head dims plus 16 columns of a tile of e4m3 ones, so that O[:, 128..143] (= the L columns) holds the
 //              row sums of the *quantised* P at no ALU cost (the reference sums P with a matrix instruction too, reduce.rs:163-173).
@@ -419,7 +419,7 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     if (warp == kKProducerWarp) {
         // This warp sets the barriers up and sends out the CTA's first copies (Q, K and V tile of its first item, their scales) while the others are still at
         // the rest of the set-up: what a launch starts with is the wait for them. From the role's own loop they went out 600 clocks later (launches in a graph:
-        // B1 H2 S256 5.83 us, so 5.42; one row block of 16 tiles 13.30 and 12.86).
+        // B1 H2 S256 5.83 us, so 5.42; one row block of 16 tiles 13.30 and 12.86; calls of the former one by one wait for the host, 7.0 us either way).
         if (lane < 3) prefetch_tmap(lane == 0 ? &tm_q : lane == 1 ? &tm_k : &tm_v);
         const uint32_t l = static_cast<uint32_t>(lane);
         uint32_t count = 1u;                                   // of barrier l (SmemLayout::bars); lanes 30 and 31: peer_rdy and peer_data
@@ -480,7 +480,8 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         }
     };
     // nothing above but the first copies, which wait for themselves, touches global memory; everything below may read what the previous grid in the stream wrote
-    // (a quantiser that is still writing the scales as this grid starts, for one): by TMA or with volatile loads, never through __ldg, which the compiler may move in front of the wait
+    // (a quantiser that is still writing the scales as this grid starts, for one): by TMA, cp.async or ld in volatile asm, which stays behind the wait, never through __ldg, which the
+    // compiler may move in front of it
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x == 0) stamp(cta_traced ? p.trace : nullptr, 2, 30, 2);   // setup done
 
@@ -495,9 +496,9 @@ mxfp8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     if (warp == kKProducerWarp || warp == kVProducerWarp) {
         // =========================================================== producers: Q, K, V tiles; Q and K scales ===========================================================
         // Warp 1 issues the Q and K tile copies and, with 4-byte asynchronous copies, their scale bytes (4 per row, strided by the head count, which a
-        // TMA box cannot express); warp 3 issues the V tile copies. Both run ahead as far as their rings go. The scales used to be loaded into registers four
-        // tiles ahead and stored by the two warps in turn: a K tile's scales then waited for the V ring on every second tile, and a launch's first tile for
-        // the loads of the first five (B1 H37 S512 Skv2048, 148 items of 16 tiles: 16.3 us, so 15.2; B4 H8 S2048 48.7, so 47.7).
+        // TMA box cannot express); warp 3 issues the V tile copies. Both run ahead as far as their rings go, and neither's tiles wait for the other's ring: with a K
+        // tile's scales behind the V ring on every second tile, as loads into registers four tiles ahead, B2 H16 HK4 S1000 Skv1337 took 21.8 us, so 19.2;
+        // B1 H8 S2048 16.5 and 14.9; B4 H8 S2048 50.7 and 49.8 (back to back; the set-up's first copies have their share in it).
         auto producer = [&](auto is_k_c) {
             constexpr bool kIsK = decltype(is_k_c)::value;
             const uint32_t tile_step = 128u * p.HK * 4u;   // of the K scales: bytes between key tiles
@@ -1597,7 +1598,9 @@ cudaError_t launch_attention(const CUtensorMap& tm_q, const CUtensorMap& tm_k, c
     // Few items: each is cut between the CTAs of a cluster, as far as the machine holds the clusters at once and it is worth it. The merge stays in shared
     // memory, with f32 partials and no workspace. What it costs, in key tiles of 0.58 us (1140 clocks at 1965 MHz): the launch as clusters
     // 8 (64 items of 4 valid rows, 16 tiles: 15.2 us whole, 15.6 us as halves; 32 tiles: 24.7 and 20.3), the exchange of 128 rows another 5 (64 items of 128 rows,
-    // 16 tiles: 15.8 and 18.2 us; 32 tiles: 25.5 and 23.3; 8 items, 16 tiles, in 16 parts: 13.9 and 13.3). Cutting only the last of several rounds this way gained
+    // 16 tiles: 15.8 and 18.2 us; 32 tiles: 25.5 and 23.3; 8 items, 16 tiles, in 16 parts: 13.9 and 13.3). With the first copies in the set-up both forms start earlier and
+    // the rule still takes the faster one: 64 items of 128 rows, 32 tiles 24.8 whole and 21.6 as halves; of 4 rows 23.0 and 18.6; 20 items, 24 tiles 17.9 and 14.6; 8 items, 16 tiles
+    // 13.2 and 12.1, 64 tiles 39.2 and 15.9. Cutting only the last of several rounds this way gained
     // 1 % at 64 tiles and lost 4 % at 16: not done.
     const bool plain = p.trace == nullptr && p.peer == nullptr && !fused && !(p.flags & (kFlagF32Partials | kFlagNoTailSplit));
     if (lazy_recipe && plain && 2u * q.n_items <= static_cast<uint32_t>(sms)) {

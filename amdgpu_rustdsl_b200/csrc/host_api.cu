@@ -448,7 +448,10 @@ int fmha_mxfp8_auto_unsplit(uint64_t b, uint64_t h, uint64_t hk, uint64_t s, uin
     uint32_t shift = 0;
     const double sms = n_sms, n = static_cast<double>(count_items(b, h, s, log2_u32(static_cast<uint32_t>(gqa)), &shift)), tiles = static_cast<double>((sk + 127) / 128);
     // us of a launch of `items` items of `len` key tiles: a start of 5.3, per round 1 for the hand-over between items, and a key tile in 0.58 with few SMs busy, 0.78 with
-    // all of them, which is what launches of 8 to 222 items of 4 to 64 tiles measured; or cut between the CTAs of clusters (launch_attention). The
+    // all of them, which is what launches of 8 to 222 items of 4 to 64 tiles measured when the start was longer; or cut between the CTAs of clusters (launch_attention). Since the
+    // first copies go out in the set-up, start and hand-over together are 4.5 and a tile is 0.54 to 0.77: 8 items of 16 tiles 13.1 us (15.7 here), of 64 tiles 39.2 (44.3), 148 items of
+    // 64 tiles 55.6 to 57.6 (56.2). Both forms are over-estimated alike, and the choice holds: of 13 dispatched splits over the path's range (1 to 8 sequences, 64 to 2048 rows, 2048 to
+    // 16384 keys) the form taken was within 2 % of the faster one. The
     // difference is the clock, not contention: a tile is 1090 to 1180 clocks with 1 to 148 items, but under the power cap all SMs together run at 1515 to 1600
     // MHz and a few at 1965. Where a box has another cap the two sides shift together; the margin of 10 % below is for that.
     const double merge = 4.6 + 2.9 * std::min(128.0, static_cast<double>(s << shift)) / 128.0;
